@@ -28,6 +28,7 @@
 // from checkpoints taken every `checkpoint_every` steps.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <string>
 #include <vector>
 
@@ -41,7 +42,7 @@ void set_error(const std::string& msg);
 namespace {
 
 template <class R>
-__device__ __forceinline__ R wR(int q) {
+__device__ __forceinline__ constexpr R wR(int q) {
     return q == 0 ? R(1) / R(3) : (q <= 6 ? R(1) / R(18) : R(1) / R(36));
 }
 
@@ -54,11 +55,75 @@ struct AdjP {
     R omega, fx, fy, fz;
 };
 
-__device__ __forceinline__ int wrapa(int v, int n) { return v < 0 ? v + n : (v >= n ? v - n : v); }
+// Every loop over the directions is unrolled, so that c_q is a literal, the 19
+// populations stay in registers and a product with c_q = 0 is no instruction.
+// With the loops rolled the arrays lived in local memory: 315 us (forward) and
+// 320 us (reverse) per 128x64x64 step in FP32, against 12 us of traffic; the
+// gradient of 100 such steps (checkpoints every 25) went from 105.6 to 17.4 ms,
+// host copies and allocations included.
+template <int C, class R>
+__device__ __forceinline__ R plus_c(R s, R v) { return C > 0 ? s + v : (C < 0 ? s - v : s); }
+// c_q . u
+template <int q, class R>
+__device__ __forceinline__ R cdot(R ux, R uy, R uz) {
+    return plus_c<cz(q)>(plus_c<cy(q)>(plus_c<cx(q)>(R(0), ux), uy), uz);
+}
+template <int q> struct QC { static constexpr int value = q; };
+template <int Q0, int Q1, class F>
+__device__ __forceinline__ void for_q(F&& fn) {
+    if constexpr (Q0 < Q1) {
+        fn(QC<Q0>{});
+        for_q<Q0 + 1, Q1>(fn);
+    }
+}
+
+// One cell and its neighbours' indices, periodic in every axis (a link past the
+// duct's ends never streams, so its index is not used).
+template <class IDX>
+struct AdjCell {
+    int x, y, z;
+    IDX row[3][3];   // [dy+1][dz+1]
+    int xs[3];
+    __device__ __forceinline__ void init(uint32_t id, int nx, int ny, int nz) {
+        const uint32_t r = id / (uint32_t)nx;
+        x = (int)(id - r * (uint32_t)nx);
+        z = (int)(r / (uint32_t)ny);
+        y = (int)(r - (uint32_t)z * (uint32_t)ny);
+        const int yy[3] = {y == 0 ? ny - 1 : y - 1, y, y == ny - 1 ? 0 : y + 1};
+        const int zz[3] = {z == 0 ? nz - 1 : z - 1, z, z == nz - 1 ? 0 : z + 1};
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+#pragma unroll
+            for (int b = 0; b < 3; ++b) row[a][b] = ((IDX)zz[b] * (IDX)ny + (IDX)yy[a]) * (IDX)nx;
+        xs[0] = x == 0 ? nx - 1 : x - 1;
+        xs[1] = x;
+        xs[2] = x == nx - 1 ? 0 : x + 1;
+    }
+    template <int q>
+    __device__ __forceinline__ IDX to() const { return row[cy(q) + 1][cz(q) + 1] + (IDX)xs[cx(q) + 1]; }
+};
 
 template <class R>
-__device__ __forceinline__ int64_t nbr(const AdjP<R>& p, int x, int y, int z, int q) {
-    return ((int64_t)wrapa(z + cz(q), p.nz) * p.ny + wrapa(y + cy(q), p.ny)) * p.nx + wrapa(x + cx(q), p.nx);
+struct AdjMom {
+    R rho, ux, uy, uz, uu;
+};
+template <class R>
+__device__ __forceinline__ AdjMom<R> adj_moments(const R (&fq)[19], const AdjP<R>& p) {
+    AdjMom<R> m;
+    R jx = 0, jy = 0, jz = 0;
+    m.rho = 0;
+    for_q<0, 19>([&](auto qi) {
+        constexpr int q = decltype(qi)::value;
+        m.rho += fq[q];
+        jx = plus_c<cx(q)>(jx, fq[q]);
+        jy = plus_c<cy(q)>(jy, fq[q]);
+        jz = plus_c<cz(q)>(jz, fq[q]);
+    });
+    m.ux = jx / m.rho + p.fx;
+    m.uy = jy / m.rho + p.fy;
+    m.uz = jz / m.rho + p.fz;
+    m.uu = m.ux * m.ux + m.uy * m.uy + m.uz * m.uz;
+    return m;
 }
 
 template <class R>
@@ -66,61 +131,69 @@ __global__ void adj_init(AdjP<R> p, const double* __restrict__ u0, R* __restrict
     for (int64_t id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; id < p.N; id += (int64_t)gridDim.x * blockDim.x) {
         const R ux = (R)u0[id], uy = (R)u0[p.N + id], uz = (R)u0[2 * p.N + id];
         const R uu = ux * ux + uy * uy + uz * uz;
-        for (int q = 0; q < 19; ++q) {
-            const R cu = (R)cx(q) * ux + (R)cy(q) * uy + (R)cz(q) * uz;
+        for_q<0, 19>([&](auto qi) {
+            constexpr int q = decltype(qi)::value;
+            const R cu = cdot<q>(ux, uy, uz);
             f[q * p.N + id] = wR<R>(q) * (R(1) + R(3) * cu + R(4.5) * cu * cu - R(1.5) * uu);
-        }
+        });
     }
 }
 
-// one push step f -> fn; per-block drag partial sums (FP64)
-template <class R>
+// one push step f -> fn, one cell per thread; drag_part (or null: the step is
+// outside the window, or recomputed) adds the block's drag sum (FP64).
+// Bound by HBM/L2: the state is read once and written once.
+template <class R, class IDX>
 __global__ void __launch_bounds__(256) adj_fwd(AdjP<R> p, const R* __restrict__ f, R* __restrict__ fn,
                                                const double* __restrict__ uin, double* __restrict__ drag_part) {
     double drag = 0.0;
-    for (int64_t id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; id < p.N; id += (int64_t)gridDim.x * blockDim.x) {
+    const IDX N = (IDX)p.N;
+    const int64_t id64 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (id64 < p.N) {
+        const IDX id = (IDX)id64;
         const uint32_t fl = p.flags[id];
-        if (fl & F_SOLID) {
-            for (int q = 0; q < 19; ++q) fn[q * p.N + id] = f[q * p.N + id];
-            continue;
-        }
-        const int x = (int)(id % p.nx);
-        const int64_t row = id / p.nx;
-        const int y = (int)(row % p.ny), z = (int)(row / p.ny);
         R fq[19];
-        R rho = 0, jx = 0, jy = 0, jz = 0;
-        for (int q = 0; q < 19; ++q) {
-            fq[q] = f[q * p.N + id];
-            rho += fq[q];
-            jx += (R)cx(q) * fq[q]; jy += (R)cy(q) * fq[q]; jz += (R)cz(q) * fq[q];
-        }
-        const R ux = jx / rho + p.fx, uy = jy / rho + p.fy, uz = jz / rho + p.fz;
-        const R uu = ux * ux + uy * uy + uz * uz;
-        R fs[19];
-        for (int q = 0; q < 19; ++q) {
-            const R cu = (R)cx(q) * ux + (R)cy(q) * uy + (R)cz(q) * uz;
-            const R feq = wR<R>(q) * rho * (R(1) + R(3) * cu + R(4.5) * cu * cu - R(1.5) * uu);
-            fs[q] = fq[q] + p.omega * (feq - fq[q]);
-        }
-        const uint32_t lk = (fl & F_SPECIAL) ? p.links[id] : 0u;
-        for (int q = 0; q < 19; ++q) {
-            if (!((lk >> q) & 1u)) {
-                fn[q * p.N + nbr(p, x, y, z, q)] = fs[q];
-                continue;
-            }
-            const int xt = x + cx(q);
-            const int o = opp(q);
-            if (xt < 0) {
-                const R u = (R)uin[(int64_t)z * p.ny + y];
-                fn[o * p.N + id] = wR<R>(q) * rho * (R(1) + R(3) * u + R(3) * u * u);
-            } else if (xt >= p.nx) {
-                fn[o * p.N + id] = fs[o];
-            } else {
-                fn[o * p.N + id] = fs[q];
-                if (p.flags[nbr(p, x, y, z, q)] & F_OBST) drag += 2.0 * cx(q) * (double)fs[q];
-            }
+        for_q<0, 19>([&](auto qi) {
+            constexpr int q = decltype(qi)::value;
+            fq[q] = f[(IDX)q * N + id];
+        });
+        if (fl & F_SOLID) {
+            for_q<0, 19>([&](auto qi) {
+                constexpr int q = decltype(qi)::value;
+                fn[(IDX)q * N + id] = fq[q];
+            });
+        } else {
+            AdjCell<IDX> c;
+            c.init((uint32_t)id64, p.nx, p.ny, p.nz);
+            const AdjMom<R> m = adj_moments(fq, p);
+            for_q<0, 19>([&](auto qi) {
+                constexpr int q = decltype(qi)::value;
+                const R cu = cdot<q>(m.ux, m.uy, m.uz);
+                const R feq = wR<R>(q) * m.rho * (R(1) + R(3) * cu + R(4.5) * cu * cu - R(1.5) * m.uu);
+                fq[q] = fq[q] + p.omega * (feq - fq[q]);
+            });
+            const uint32_t lk = (fl & F_SPECIAL) ? p.links[id] : 0u;
+            for_q<0, 19>([&](auto qi) {
+                constexpr int q = decltype(qi)::value;
+                constexpr int o = opp(q);
+                const IDX t = c.template to<q>();
+                if (!((lk >> q) & 1u)) {
+                    fn[(IDX)q * N + t] = fq[q];
+                } else {
+                    R v = fq[q];
+                    if (cx(q) < 0 && c.x == 0) {
+                        const R u = (R)uin[(int64_t)c.z * p.ny + c.y];
+                        v = wR<R>(q) * m.rho * (R(1) + R(3) * u + R(3) * u * u);
+                    } else if (cx(q) > 0 && c.x == p.nx - 1) {
+                        v = fq[o];
+                    } else if (cx(q) != 0 && drag_part && (p.flags[t] & F_OBST)) {
+                        drag += 2.0 * cx(q) * (double)fq[q];
+                    }
+                    fn[(IDX)o * N + id] = v;
+                }
+            });
         }
     }
+    if (!drag_part) return;
     __shared__ double red[8];
     for (int o = 16; o > 0; o >>= 1) drag += __shfl_down_sync(0xffffffffu, drag, o);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = drag;
@@ -128,75 +201,112 @@ __global__ void __launch_bounds__(256) adj_fwd(AdjP<R> p, const R* __restrict__ 
     if (threadIdx.x == 0) {
         double s = 0.0;
         for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += red[w];
-        drag_part[blockIdx.x] = s;
+        drag_part[blockIdx.x] += s;
     }
 }
 
-// one reverse step: lam0 = (d f'/d f)^T lam1 (+ the drag term when wdrag != 0)
-template <class R>
+// out = the sum of n values in a fixed order (one block)
+__global__ void __launch_bounds__(1024) adj_sum(const double* __restrict__ v, int64_t n, double* __restrict__ out) {
+    double s = 0.0;
+    for (int64_t i = threadIdx.x; i < n; i += blockDim.x) s += v[i];
+    __shared__ double red[32];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        s = red[threadIdx.x];
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+        if (threadIdx.x == 0) *out = s;
+    }
+}
+
+// one reverse step, one cell per thread: lam0 = (d f'/d f)^T lam1 (+ the drag
+// term when wdrag != 0).  Bound by HBM/L2: f and lam1 read, lam0 written.
+template <class R, class IDX>
 __global__ void __launch_bounds__(256) adj_bwd(AdjP<R> p, const R* __restrict__ f, const R* __restrict__ lam1,
                                                R* __restrict__ lam0, const double* __restrict__ uin,
                                                double* __restrict__ g_uin, R wdrag) {
-    for (int64_t id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; id < p.N; id += (int64_t)gridDim.x * blockDim.x) {
-        const uint32_t fl = p.flags[id];
-        if (fl & F_SOLID) {
-            for (int q = 0; q < 19; ++q) lam0[q * p.N + id] = R(0);
-            continue;
-        }
-        const int x = (int)(id % p.nx);
-        const int64_t row = id / p.nx;
-        const int y = (int)(row % p.ny), z = (int)(row / p.ny);
-        R fq[19];
-        R rho = 0, jx = 0, jy = 0, jz = 0;
-        for (int q = 0; q < 19; ++q) {
-            fq[q] = f[q * p.N + id];
-            rho += fq[q];
-            jx += (R)cx(q) * fq[q]; jy += (R)cy(q) * fq[q]; jz += (R)cz(q) * fq[q];
-        }
-        const R ux = jx / rho + p.fx, uy = jy / rho + p.fy, uz = jz / rho + p.fz;
-        const R uu = ux * ux + uy * uy + uz * uz;
-        const uint32_t lk = (fl & F_SPECIAL) ? p.links[id] : 0u;
-        R ls[19];
-        for (int q = 0; q < 19; ++q) ls[q] = R(0);
-        R a_in = 0;
-        double g_in = 0.0;
-        for (int q = 0; q < 19; ++q) {
-            if (!((lk >> q) & 1u)) {
-                ls[q] += lam1[q * p.N + nbr(p, x, y, z, q)];
-                continue;
-            }
-            const int xt = x + cx(q);
-            const int o = opp(q);
-            const R lo = lam1[o * p.N + id];
-            if (xt < 0) {
-                const R u = (R)uin[(int64_t)z * p.ny + y];
-                a_in += lo * wR<R>(q) * (R(1) + R(3) * u + R(3) * u * u);
-                g_in += (double)(lo * wR<R>(q) * rho * (R(3) + R(6) * u));
-            } else if (xt >= p.nx) {
-                ls[o] += lo;
-            } else {
-                ls[q] += lo;
-                if (wdrag != R(0) && (p.flags[nbr(p, x, y, z, q)] & F_OBST)) ls[q] += wdrag * R(2 * cx(q));
-            }
-        }
-        if (x == 0 && g_uin) g_uin[(int64_t)z * p.ny + y] += g_in;
-        R A = 0, Bx = 0, By = 0, Bz = 0;
-        for (int q = 0; q < 19; ++q) {
-            const R cu = (R)cx(q) * ux + (R)cy(q) * uy + (R)cz(q) * uz;
-            const R w = wR<R>(q);
-            A += ls[q] * w * (R(1) + R(3) * cu + R(4.5) * cu * cu - R(1.5) * uu);
-            const R t = ls[q] * w * rho;
-            Bx += t * (R(3) * cx(q) + R(9) * cu * cx(q) - R(3) * ux);
-            By += t * (R(3) * cy(q) + R(9) * cu * cy(q) - R(3) * uy);
-            Bz += t * (R(3) * cz(q) + R(9) * cu * cz(q) - R(3) * uz);
-        }
-        const R om = p.omega;
-        const R vx = ux - p.fx, vy = uy - p.fy, vz = uz - p.fz;
-        for (int q = 0; q < 19; ++q) {
-            const R du = (Bx * ((R)cx(q) - vx) + By * ((R)cy(q) - vy) + Bz * ((R)cz(q) - vz)) / rho;
-            lam0[q * p.N + id] = (R(1) - om) * ls[q] + om * (A + du) + a_in;
-        }
+    const IDX N = (IDX)p.N;
+    const int64_t id64 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (id64 >= p.N) return;
+    const IDX id = (IDX)id64;
+    const uint32_t fl = p.flags[id];
+    if (fl & F_SOLID) {
+        for_q<0, 19>([&](auto qi) {
+            constexpr int q = decltype(qi)::value;
+            lam0[(IDX)q * N + id] = R(0);
+        });
+        return;
     }
+    AdjCell<IDX> c;
+    c.init((uint32_t)id64, p.nx, p.ny, p.nz);
+    AdjMom<R> m;
+    {
+        R fq[19];
+        for_q<0, 19>([&](auto qi) {
+            constexpr int q = decltype(qi)::value;
+            fq[q] = f[(IDX)q * N + id];
+        });
+        m = adj_moments(fq, p);
+    }
+    const uint32_t lk = (fl & F_SPECIAL) ? p.links[id] : 0u;
+    R ls[19];
+    R a_in = 0;
+    // what arrives over each link: a streaming one from the neighbour, another
+    // from the cell's own slot opp(q)
+    for_q<0, 19>([&](auto qi) {
+        constexpr int q = decltype(qi)::value;
+        constexpr int o = opp(q);
+        const bool nn = (lk >> q) & 1u;
+        ls[q] = lam1[nn ? (IDX)o * N + id : (IDX)q * N + c.template to<q>()];
+    });
+    if (lk) {
+        double g_in = 0.0;
+        R keep[19];      // outlet copies, added once every direction is resolved
+        for_q<0, 19>([&](auto qi) {
+            constexpr int q = decltype(qi)::value;
+            constexpr int o = opp(q);
+            keep[o] = 0;
+            if ((lk >> q) & 1u) {
+                const R lo = ls[q];
+                if (cx(q) < 0 && c.x == 0) {
+                    const R u = (R)uin[(int64_t)c.z * p.ny + c.y];
+                    a_in += lo * wR<R>(q) * (R(1) + R(3) * u + R(3) * u * u);
+                    g_in += (double)(lo * wR<R>(q) * m.rho * (R(3) + R(6) * u));
+                    ls[q] = 0;
+                } else if (cx(q) > 0 && c.x == p.nx - 1) {
+                    keep[o] = lo;
+                    ls[q] = 0;
+                } else if (cx(q) != 0 && wdrag != R(0) && (p.flags[c.template to<q>()] & F_OBST)) {
+                    ls[q] += wdrag * R(2 * cx(q));
+                }
+            }
+        });
+        for_q<0, 19>([&](auto qi) {
+            constexpr int q = decltype(qi)::value;
+            ls[q] += keep[q];
+        });
+        if (c.x == 0 && g_uin) g_uin[(int64_t)c.z * p.ny + c.y] += g_in;
+    }
+    R A = 0, Bx = 0, By = 0, Bz = 0;
+    for_q<0, 19>([&](auto qi) {
+        constexpr int q = decltype(qi)::value;
+        const R cu = cdot<q>(m.ux, m.uy, m.uz);
+        const R w = wR<R>(q);
+        A += ls[q] * w * (R(1) + R(3) * cu + R(4.5) * cu * cu - R(1.5) * m.uu);
+        const R t = ls[q] * w * m.rho;
+        const R k = R(3) + R(9) * cu;     // 3 + 9 c.u
+        Bx += t * plus_c<cx(q)>(-R(3) * m.ux, k);
+        By += t * plus_c<cy(q)>(-R(3) * m.uy, k);
+        Bz += t * plus_c<cz(q)>(-R(3) * m.uz, k);
+    });
+    const R om = p.omega;
+    const R gx = Bx / m.rho, gy = By / m.rho, gz = Bz / m.rho;
+    const R base = om * (A - (gx * (m.ux - p.fx) + gy * (m.uy - p.fy) + gz * (m.uz - p.fz))) + a_in;
+    for_q<0, 19>([&](auto qi) {
+        constexpr int q = decltype(qi)::value;
+        lam0[(IDX)q * N + id] = (R(1) - om) * ls[q] + (om * cdot<q>(gx, gy, gz) + base);
+    });
 }
 
 template <class R>
@@ -204,24 +314,22 @@ __global__ void adj_grad_u0(AdjP<R> p, const double* __restrict__ u0, const R* _
     for (int64_t id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; id < p.N; id += (int64_t)gridDim.x * blockDim.x) {
         const R ux = (R)u0[id], uy = (R)u0[p.N + id], uz = (R)u0[2 * p.N + id];
         R gx = 0, gy = 0, gz = 0;
-        for (int q = 0; q < 19; ++q) {
-            const R cu = (R)cx(q) * ux + (R)cy(q) * uy + (R)cz(q) * uz;
+        for_q<0, 19>([&](auto qi) {
+            constexpr int q = decltype(qi)::value;
+            const R cu = cdot<q>(ux, uy, uz);
             const R t = lam[q * p.N + id] * wR<R>(q);
-            gx += t * (R(3) * cx(q) + R(9) * cu * cx(q) - R(3) * ux);
-            gy += t * (R(3) * cy(q) + R(9) * cu * cy(q) - R(3) * uy);
-            gz += t * (R(3) * cz(q) + R(9) * cu * cz(q) - R(3) * uz);
-        }
+            const R k = R(3) + R(9) * cu;
+            gx += t * plus_c<cx(q)>(-R(3) * ux, k);
+            gy += t * plus_c<cy(q)>(-R(3) * uy, k);
+            gz += t * plus_c<cz(q)>(-R(3) * uz, k);
+        });
         g[id] = (double)gx;
         g[p.N + id] = (double)gy;
         g[2 * p.N + id] = (double)gz;
     }
 }
 
-int grid_of(int64_t n) {
-    const int64_t b = (n + 255) / 256;
-    const int64_t cap = (int64_t)num_sms() * 8;
-    return (int)(b < 1 ? 1 : (b > cap ? cap : b));
-}
+int blocks_for(int64_t n) { return (int)((n + 255) / 256); }
 
 #define ACK(call)                                                                          \
     do {                                                                                   \
@@ -247,6 +355,20 @@ struct AdjBuffers {
 };
 
 template <class R>
+void run_fwd(const AdjP<R>& p, const R* f, R* fn, const double* uin, double* drag, cudaStream_t s) {
+    // 32-bit element offsets while every slot index 19*N fits in them
+    if ((uint64_t)p.N * 19u < (1ull << 32)) adj_fwd<R, uint32_t><<<blocks_for(p.N), 256, 0, s>>>(p, f, fn, uin, drag);
+    else adj_fwd<R, int64_t><<<blocks_for(p.N), 256, 0, s>>>(p, f, fn, uin, drag);
+}
+template <class R>
+void run_bwd(const AdjP<R>& p, const R* f, const R* lam1, R* lam0, const double* uin, double* guin, R wd,
+             cudaStream_t s) {
+    if ((uint64_t)p.N * 19u < (1ull << 32))
+        adj_bwd<R, uint32_t><<<blocks_for(p.N), 256, 0, s>>>(p, f, lam1, lam0, uin, guin, wd);
+    else adj_bwd<R, int64_t><<<blocks_for(p.N), 256, 0, s>>>(p, f, lam1, lam0, uin, guin, wd);
+}
+
+template <class R>
 int adjoint_run(const lbm_adj_problem* pr, const uint8_t* flags, const uint32_t* links, const double* h_uin,
                 const double* h_u0, double* J, double* h_g_uin, double* h_g_u0, cudaStream_t s) {
     const int64_t N = (int64_t)pr->nx * pr->ny * pr->nz;
@@ -257,67 +379,75 @@ int adjoint_run(const lbm_adj_problem* pr, const uint8_t* flags, const uint32_t*
     const bool want_grad = h_g_uin || h_g_u0;
     AdjP<R> p{flags, links, pr->nx, pr->ny, pr->nz, N, R(1) / (R)pr->tau, (R)pr->force[0], (R)pr->force[1],
               (R)pr->force[2]};
-    const int grid = grid_of(N);
+    const int grid = blocks_for(N);
+    const int small = grid < num_sms() * 8 ? grid : num_sms() * 8;   // the set-up kernels stride over the cells
     AdjBuffers B;
-    double *d_uin = nullptr, *d_u0 = nullptr, *d_drag = nullptr, *d_guin = nullptr, *d_gu0 = nullptr;
+    double *d_uin = nullptr, *d_u0 = nullptr, *d_drag = nullptr, *d_J = nullptr, *d_guin = nullptr, *d_gu0 = nullptr;
     R *fa = nullptr, *fb = nullptr;
-    const int nseg = (steps + K - 1) / K;
-    R* ckpt = nullptr;     // f^{kK}, k = 0 .. nseg-1
-    R* seg = nullptr;      // f^{sK} .. f^{sK+K-1} of the segment being reversed
-    bool ok = B.alloc(&d_uin, NI) && B.alloc(&d_u0, 3 * N) && B.alloc(&d_drag, (size_t)grid * (steps + 1)) &&
-              B.alloc(&fa, 19 * N) && B.alloc(&fb, 19 * N);
+    const int nseg = (steps - 1) / K + 1;
+    const int last0 = (nseg - 1) * K;                 // first state of the last segment
+    const size_t state = 19 * (size_t)N;
+    const int inner = std::min(K, steps) - 1;         // states of a segment behind its checkpoint
+    R* ckpt = nullptr;     // f^{kK}, k = 0 .. nseg-1, written there by the step that produces them
+    R* seg = nullptr;      // f^{n0+1} .. f^{n0+inner} of the segment being reversed
+    bool ok = B.alloc(&d_uin, NI) && B.alloc(&d_u0, 3 * N) && B.alloc(&d_drag, grid) && B.alloc(&d_J, 1) &&
+              B.alloc(&fa, state) && B.alloc(&fb, state);
     if (want_grad)
-        ok = ok && B.alloc(&ckpt, (size_t)nseg * 19 * N) && B.alloc(&seg, (size_t)K * 19 * N) &&
+        ok = ok && B.alloc(&ckpt, (size_t)nseg * state) && B.alloc(&seg, (size_t)inner * state) &&
              B.alloc(&d_guin, NI) && B.alloc(&d_gu0, 3 * N);
     if (!ok) { set_error("lbm_adjoint: device allocation failed"); return LBM_ERR_ALLOC; }
+    auto seg_state = [&](int k, int j) { return j == 0 ? ckpt + (size_t)k * state : seg + (size_t)(j - 1) * state; };
     ACK(cudaMemcpyAsync(d_uin, h_uin, sizeof(double) * NI, cudaMemcpyHostToDevice, s));
     ACK(cudaMemcpyAsync(d_u0, h_u0, sizeof(double) * 3 * N, cudaMemcpyHostToDevice, s));
-    adj_init<R><<<grid, 256, 0, s>>>(p, d_u0, fa);
+    ACK(cudaMemsetAsync(d_drag, 0, sizeof(double) * grid, s));
+    R* cur = want_grad ? ckpt : fa;
+    adj_init<R><<<small, 256, 0, s>>>(p, d_u0, cur);
     ACK(cudaGetLastError());
-    // forward: f^{n-1} -> f^n, drag of step n in d_drag[n * grid ...]
+    // forward: f^{n-1} -> f^n.  Checkpoints and the last segment's states are
+    // written where the reverse pass reads them, so nothing is copied and the
+    // last segment is not recomputed; the drag of the window's steps adds up in d_drag.
     for (int n = 1; n <= steps; ++n) {
-        if (want_grad && (n - 1) % K == 0)
-            ACK(cudaMemcpyAsync(ckpt + (size_t)((n - 1) / K) * 19 * N, fa, sizeof(R) * 19 * N,
-                                cudaMemcpyDeviceToDevice, s));
-        adj_fwd<R><<<grid, 256, 0, s>>>(p, fa, fb, d_uin, d_drag + (size_t)n * grid);
+        R* dst = cur == fa ? fb : fa;
+        if (want_grad && n < steps) {
+            if (n % K == 0) dst = seg_state(n / K, 0);
+            else if (n > last0) dst = seg_state(nseg - 1, n - last0);
+        }
+        run_fwd<R>(p, cur, dst, d_uin, n >= wb && n <= we ? d_drag : nullptr, s);
         ACK(cudaGetLastError());
-        std::swap(fa, fb);
+        cur = dst;
     }
-    std::vector<double> drag((size_t)grid * (steps + 1));
-    ACK(cudaMemcpyAsync(drag.data(), d_drag, sizeof(double) * drag.size(), cudaMemcpyDeviceToHost, s));
-    ACK(cudaStreamSynchronize(s));
-    double acc = 0.0;
-    for (int n = wb; n <= we; ++n)
-        for (int b = 0; b < grid; ++b) acc += drag[(size_t)n * grid + b];
-    *J = acc / nwin;
-    if (!want_grad) return LBM_OK;
-
-    // reverse: lambda^steps = 0; lambda^{n-1} from lambda^n and f^{n-1}
-    R* lam1 = fa;
-    R* lam0 = fb;
-    ACK(cudaMemsetAsync(lam1, 0, sizeof(R) * 19 * N, s));
-    ACK(cudaMemsetAsync(d_guin, 0, sizeof(double) * NI, s));
-    for (int sgi = nseg - 1; sgi >= 0; --sgi) {
-        const int n0 = sgi * K;                          // f^{n0} is the checkpoint
-        const int n1 = std::min(steps, n0 + K);          // states f^{n0} .. f^{n1-1} are needed
-        ACK(cudaMemcpyAsync(seg, ckpt + (size_t)sgi * 19 * N, sizeof(R) * 19 * N, cudaMemcpyDeviceToDevice, s));
-        for (int n = n0 + 1; n < n1; ++n) {
-            adj_fwd<R><<<grid, 256, 0, s>>>(p, seg + (size_t)(n - 1 - n0) * 19 * N, seg + (size_t)(n - n0) * 19 * N,
-                                            d_uin, d_drag);
-            ACK(cudaGetLastError());
-        }
-        for (int n = n1; n > n0; --n) {
-            const R wd = (n >= wb && n <= we) ? R(1) / (R)nwin : R(0);
-            adj_bwd<R><<<grid, 256, 0, s>>>(p, seg + (size_t)(n - 1 - n0) * 19 * N, lam1, lam0, d_uin, d_guin, wd);
-            ACK(cudaGetLastError());
-            std::swap(lam0, lam1);
-        }
-    }
-    adj_grad_u0<R><<<grid, 256, 0, s>>>(p, d_u0, lam1, d_gu0);
+    adj_sum<<<1, 1024, 0, s>>>(d_drag, grid, d_J);
     ACK(cudaGetLastError());
-    if (h_g_uin) ACK(cudaMemcpyAsync(h_g_uin, d_guin, sizeof(double) * NI, cudaMemcpyDeviceToHost, s));
-    if (h_g_u0) ACK(cudaMemcpyAsync(h_g_u0, d_gu0, sizeof(double) * 3 * N, cudaMemcpyDeviceToHost, s));
+    double acc = 0.0;
+    ACK(cudaMemcpyAsync(&acc, d_J, sizeof(double), cudaMemcpyDeviceToHost, s));
+    if (want_grad) {
+        // reverse: lambda^steps = 0; lambda^{n-1} from lambda^n and f^{n-1}
+        R* lam1 = fa;
+        R* lam0 = fb;
+        ACK(cudaMemsetAsync(lam1, 0, sizeof(R) * state, s));
+        ACK(cudaMemsetAsync(d_guin, 0, sizeof(double) * NI, s));
+        for (int k = nseg - 1; k >= 0; --k) {
+            const int n0 = k * K;                            // f^{n0} is the checkpoint
+            const int n1 = std::min(steps, n0 + K);          // states f^{n0} .. f^{n1-1} are needed
+            if (k < nseg - 1)
+                for (int j = 1; j < n1 - n0; ++j) {
+                    run_fwd<R>(p, seg_state(k, j - 1), seg_state(k, j), d_uin, nullptr, s);
+                    ACK(cudaGetLastError());
+                }
+            for (int n = n1; n > n0; --n) {
+                const R wd = (n >= wb && n <= we) ? R(1) / (R)nwin : R(0);
+                run_bwd<R>(p, seg_state(k, n - 1 - n0), lam1, lam0, d_uin, d_guin, wd, s);
+                ACK(cudaGetLastError());
+                std::swap(lam0, lam1);
+            }
+        }
+        adj_grad_u0<R><<<small, 256, 0, s>>>(p, d_u0, lam1, d_gu0);
+        ACK(cudaGetLastError());
+        if (h_g_uin) ACK(cudaMemcpyAsync(h_g_uin, d_guin, sizeof(double) * NI, cudaMemcpyDeviceToHost, s));
+        if (h_g_u0) ACK(cudaMemcpyAsync(h_g_u0, d_gu0, sizeof(double) * 3 * N, cudaMemcpyDeviceToHost, s));
+    }
     ACK(cudaStreamSynchronize(s));
+    *J = acc / nwin;
     return LBM_OK;
 }
 

@@ -74,6 +74,33 @@ def test_checkpoint_interval_does_not_change_the_gradient(gpu, tiny):
         np.testing.assert_array_equal(gu, ref[2])
 
 
+@pytest.mark.parametrize("dims,steps,window,every", [
+    ((19, 7, 5), 9, (4, 9), 4),        # ragged last block, ragged last segment
+    ((3, 16, 16), 6, (1, 6), 6),       # the shortest duct: inlet and outlet cells only one apart
+    ((33, 5, 9), 1, (1, 1), 3),        # one step, checkpoint interval past the end
+    ((40, 1, 16), 7, (7, 7), 1),       # one row in y (it wraps onto itself), every state a checkpoint
+])
+def test_ragged_grids_match_fp64_autodiff(gpu, dims, steps, window, every):
+    """Sizes at the edges of the blocks and segments, FP64, with the bounds of the 32x16x16 case."""
+    import torch
+    from torch_duct import TorchDuct
+    nx, ny, nz = dims
+    mask = np.zeros((nz, ny, nx), np.uint8)
+    mask[nz // 2, ny // 2, nx // 2] = W.MASK_SOLID
+    mask[0, :, :] = W.MASK_SOLID | W.MASK_WALL
+    ui, u0 = controls(nx, ny, nz, 3)
+    prob = DuctProblem(nx, ny, nz, 0.6, mask, n_steps=steps, window=window, checkpoint_every=every)
+    tui = torch.tensor(ui, requires_grad=True)
+    tu0 = torch.tensor(u0, requires_grad=True)
+    Jt = TorchDuct(mask, 0.6).objective(tui, tu0, steps, window)
+    Jt.backward()
+    J, gi, gu = objective(prob, ui, u0, "f64", grad=True)
+    assert J == pytest.approx(Jt.item(), rel=1e-11)
+    ti = np.zeros((nz, ny)) if tui.grad is None else tui.grad.numpy()    # one step: no inlet value is read
+    for a, b in ((gi, ti), (gu, tu0.grad.numpy())):
+        assert np.linalg.norm(a - b) <= 1e-9 * np.linalg.norm(b)
+
+
 def test_adjoint_matches_central_differences(gpu):
     """A 64x32x32 copy of the adjoint case (sphere r=5 at (16,16,16)), 120 steps,
     drag averaged over steps 100-120: directional derivatives along random
