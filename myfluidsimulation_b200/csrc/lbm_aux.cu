@@ -121,6 +121,16 @@ __global__ void build_flags(const uint8_t* __restrict__ mask, const uint8_t* __r
                 }
             }
             if (lk) fl |= F_SPECIAL;
+            if (mask) {
+                const int64_t pl = (int64_t)nx * ny;
+                uint32_t far = 0;
+                if (mask[id + (int64_t)((y + 2) % ny - y) * nx]) far |= LK_YP2;
+                if (mask[id + (int64_t)((y + 2 * ny - 2) % ny - y) * nx]) far |= LK_YM2;
+                if (mask[id + ((z + 2) % nz - z) * pl]) far |= LK_ZP2;
+                if (mask[id + ((z + 2 * nz - 2) % nz - z) * pl]) far |= LK_ZM2;
+                if (far) fl |= F_NEAR2;
+                lk |= far;
+            }
             if (touch) fl |= F_TOUCH;
         }
         flags[id] = fl;

@@ -97,7 +97,11 @@ enum : uint8_t {
     F_OBST = 4,      // solid cell that counts for the drag (not a wall)
     F_SPECIAL = 8,   // fluid cell with at least one non-streaming link
     F_TOUCH = 16,    // fluid cell with a link into an obstacle cell
+    F_NEAR2 = 32,    // fluid cell with a solid cell two rows or planes away (LK_* in its link word)
 };
+// link word: bit q (1..18) for a link x -> x+c_q that does not stream, and whether
+// the cells at (0, +-2, 0) and (0, 0, +-2) are solid (the reference's bounce table)
+enum : uint32_t { LK_YP2 = 1u << 20, LK_YM2 = 1u << 21, LK_ZP2 = 1u << 22, LK_ZM2 = 1u << 23 };
 
 // The Legacy equilibrium, written as src/lbm/lbm3d_legacy.cu:54-58 writes it
 // (the same expression keeps nvcc's contraction pattern, hence the results, close).

@@ -164,6 +164,20 @@ def test_hybrid_vs_oracle(gpu, oracle, omega_s, bounce):
     assert vel_err(g["macros"][1:], mac[1:]) < TOL_F
 
 
+@pytest.mark.parametrize("dims", [(33, 4, 5), (5, 3, 4), (257, 2, 3), (7, 6, 2), (64, 1, 8)])
+def test_reference_bounce_small_extents_vs_oracle(gpu, oracle, dims):
+    """Extents at which the cells two rows or planes away wrap onto each other or onto the cell itself, and
+    cell counts that leave a part of the last block."""
+    fields = init_fields(*dims, seed=21)
+    mask = obstacle_mask(*dims, seed=22)
+    assert 0 < mask.sum() < mask.size
+    g = run_gpu(METHOD_LEGACY, dims, 0.6, fields, mask, 5, force=(1e-5, 0, 0), bounce=BOUNCE_REFERENCE)
+    f, mac, _ = oracle_bgk(oracle, dims, 0.6, fields, mask, 5, (1e-5, 0, 0), bb=BOUNCE_REFERENCE)
+    assert rl2(g["state"], f) < TOL_F
+    assert rl2(g["macros"][0], mac[0]) < TOL_F
+    assert vel_err(g["macros"][1:], mac[1:]) < TOL_F
+
+
 def test_hybrid_equals_legacy_by_default(gpu):
     """omega_s = omega_h makes the two collision forms the same arithmetic (hybrid.cu:264-267)."""
     dims = (16, 12, 10)
