@@ -206,8 +206,28 @@ static int wait_pending_read(lbm_solver* s) {
     return LBM_OK;
 }
 
+// Four plain steps as two two-step launches, f -> f2 -> f: the state ends in
+// the buffer it started from, so nothing outside the step sees the second one.
+static int enqueue_pairs(lbm_solver* s) {
+    const lbm::AAParams p = aa_params(s, false, false);
+    float* f = static_cast<float*>(s->f);
+    float* g = static_cast<float*>(s->f2);
+    const int zc = lbm::pair_zchunk(s->dom.nx, s->dom.ny, s->dom.nz, s->storage);
+    CK(lbm::launch_aa_pair(p, f, g, zc, s->stream));
+    CK(lbm::launch_aa_pair(p, g, f, zc, s->stream));
+    return LBM_OK;
+}
+
 static int enqueue_steps(lbm_solver* s, int n) {
     for (int i = 0; i < n; ++i) {
+        // steps behind an odd parity and before one that writes macro fields or statistics
+        while (is_aa(s) && !is_ref_push(s) && s->f2 && !s->use_flags && !s->zghost && s->parity == 1 &&
+               n - i - (s->macro_out || s->stats_on ? 1 : 0) >= 4) {
+            const int rc = enqueue_pairs(s);
+            if (rc != LBM_OK) return rc;
+            i += 4;
+        }
+        if (i == n) break;
         const bool last = (i == n - 1);
         const bool st = last && s->stats_on;
         const bool mac = last && (s->macro_out || st);
@@ -391,7 +411,7 @@ int lbm_create(const lbm_domain* dom, const lbm_options* opts, lbm_solver** out)
     bool ok = true;
     if (is_aa(s)) ok = ok && dmalloc(&s->f, s->esize * 19 * (size_t)N);
     if (is_ref_push(s)) ok = ok && dmalloc(&s->f2, s->esize * 19 * (size_t)N);
-    else ok = ok && dmalloc(&s->m[0], s->esize * 10 * (size_t)N) && dmalloc(&s->m[1], s->esize * 10 * (size_t)N);
+    if (!is_aa(s)) ok = ok && dmalloc(&s->m[0], s->esize * 10 * (size_t)N) && dmalloc(&s->m[1], s->esize * 10 * (size_t)N);
     if (is_aa(s) || s->storage != LBM_STORE_F32) ok = ok && dmalloc((void**)&s->macro, sizeof(float) * 4 * (size_t)N);
     ok = ok && dmalloc((void**)&s->mask, (size_t)N) && dmalloc((void**)&s->band, (size_t)N) &&
          dmalloc((void**)&s->flags, (size_t)N) && dmalloc((void**)&s->links, sizeof(uint32_t) * (size_t)N) &&
@@ -405,9 +425,19 @@ int lbm_create(const lbm_domain* dom, const lbm_options* opts, lbm_solver** out)
     if (cudaMemsetAsync(s->mask, 0, (size_t)N, s->stream) != cudaSuccess ||
         cudaMemsetAsync(s->band, 0, (size_t)N, s->stream) != cudaSuccess ||
         cudaMemsetAsync(s->stats, 0, sizeof(double) * lbm::NSTAT, s->stream) != cudaSuccess ||
-        (s->f2 && cudaMemsetAsync(s->f2, 0, s->esize * 19 * (size_t)N, s->stream) != cudaSuccess)) {
+        (is_ref_push(s) && cudaMemsetAsync(s->f2, 0, s->esize * 19 * (size_t)N, s->stream) != cudaSuccess)) {
         set_error("lbm_create: cudaMemset failed");
         return fail(LBM_ERR_CUDA);
+    }
+    // the second buffer of the two-step kernel; without it every step is a single one
+    if (is_aa(s) && !is_ref_push(s) && lbm::pair_zchunk(dom->nx, dom->ny, dom->nz, o.storage) > 0) {
+        if (!dmalloc(&s->f2, s->esize * 19 * (size_t)N)) {
+            cudaGetLastError();
+            s->f2 = nullptr;
+        } else if (lbm::pair_prepare() != cudaSuccess) {
+            set_error("lbm_create: cannot set the two-step kernel's shared-memory size");
+            return fail(LBM_ERR_CUDA);
+        }
     }
     if (!is_aa(s) && lbm::home_prepare() != cudaSuccess) {
         set_error("lbm_create: cannot set the HOME kernel's shared-memory size");

@@ -40,6 +40,7 @@
 
 #include "lbm_common.cuh"
 #include "lbm_internal.h"
+#include "lbm_vec.cuh"
 
 namespace lbm {
 namespace {
@@ -80,37 +81,6 @@ struct Ring {
     }
 };
 
-// ---- scalar and paired FP32 arithmetic with identical rounding -------------
-__device__ __forceinline__ float vadd(float a, float b) { return __fadd_rn(a, b); }
-__device__ __forceinline__ float vsub(float a, float b) { return __fsub_rn(a, b); }
-__device__ __forceinline__ float vmul(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ float vfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-__device__ __forceinline__ float vsplat(float s, float) { return s; }
-__device__ __forceinline__ float2 vadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ float2 vsub(float2 a, float2 b) { return __fadd2_rn(a, make_float2(-b.x, -b.y)); }
-__device__ __forceinline__ float2 vmul(float2 a, float2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ float2 vfma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-__device__ __forceinline__ float2 vsplat(float s, float2) { return make_float2(s, s); }
-// FP64 (the reference form): one double, or a pair of doubles with the same
-// interface as float2
-struct D2 {
-    double x, y;
-};
-__device__ __forceinline__ double vadd(double a, double b) { return __dadd_rn(a, b); }
-__device__ __forceinline__ double vsub(double a, double b) { return __dsub_rn(a, b); }
-__device__ __forceinline__ double vmul(double a, double b) { return __dmul_rn(a, b); }
-__device__ __forceinline__ double vfma(double a, double b, double c) { return __fma_rn(a, b, c); }
-__device__ __forceinline__ double vsplat(float s, double) { return s; }
-__device__ __forceinline__ D2 vadd(D2 a, D2 b) { return {__dadd_rn(a.x, b.x), __dadd_rn(a.y, b.y)}; }
-__device__ __forceinline__ D2 vsub(D2 a, D2 b) { return {__dsub_rn(a.x, b.x), __dsub_rn(a.y, b.y)}; }
-__device__ __forceinline__ D2 vmul(D2 a, D2 b) { return {__dmul_rn(a.x, b.x), __dmul_rn(a.y, b.y)}; }
-__device__ __forceinline__ D2 vfma(D2 a, D2 b, D2 c) { return {__fma_rn(a.x, b.x, c.x), __fma_rn(a.y, b.y, c.y)}; }
-__device__ __forceinline__ D2 vsplat(float s, D2) { return {(double)s, (double)s}; }
-__device__ __forceinline__ D2 vsplat(double s, D2) { return {s, s}; }
-__device__ __forceinline__ double vsplat(double s, double) { return s; }
-using lbm::mulk;   // the float, float2 and double forms, next to the pair of doubles below
-__device__ __forceinline__ D2 mulk(D2 x, float hi, float lo) { return {lbm::mulk(x.x, hi, lo), lbm::mulk(x.y, hi, lo)}; }
-
 // element type of the ring and of one cell's arithmetic (E), and of a pair (V)
 template <class T> struct HomeTypes {
     using E = float;
@@ -120,19 +90,6 @@ template <> struct HomeTypes<double> {
     using E = double;
     using V = D2;
 };
-// one aligned pair in shared memory
-__device__ __forceinline__ void st_pair(float* p, float2 v) { *reinterpret_cast<float2*>(p) = v; }
-__device__ __forceinline__ void st_pair(double* p, D2 v) { *reinterpret_cast<double2*>(p) = make_double2(v.x, v.y); }
-__device__ __forceinline__ float2 ld_pair(const float* p) { return *reinterpret_cast<const float2*>(p); }
-__device__ __forceinline__ D2 ld_pair(const double* p) {
-    const double2 v = *reinterpret_cast<const double2*>(p);
-    return {v.x, v.y};
-}
-// 1/r where r > 0, else 0 (u = 0 for an empty cell, home.cu:258-262)
-__device__ __forceinline__ float2 vrcp_pos(float2 r) {
-    return make_float2(r.x > 0.f ? __frcp_rn(r.x) : 0.f, r.y > 0.f ? __frcp_rn(r.y) : 0.f);
-}
-__device__ __forceinline__ D2 vrcp_pos(D2 r) { return {r.x > 0.0 ? 1.0 / r.x : 0.0, r.y > 0.0 ? 1.0 / r.y : 0.0}; }
 // the inlet population of a direction with c_x = +1, shifted by w_q rho0:
 // feq(rho, (u_in, 0, 0)) - w_q rho0 (src/lbm/lbm3d_legacy.cu:54-58 form)
 template <int q>

@@ -178,6 +178,23 @@ def test_reference_bounce_small_extents_vs_oracle(gpu, oracle, dims):
     assert vel_err(g["macros"][1:], mac[1:]) < TOL_F
 
 
+@pytest.mark.parametrize("dims", [(32, 8, 5), (33, 9, 7), (31, 7, 1), (64, 24, 49), (66, 17, 2), (3, 3, 3), (1, 1, 4),
+                                  (2, 40, 16), (100, 50, 6)])
+@pytest.mark.parametrize("method", [METHOD_LEGACY, METHOD_HYBRID])
+def test_two_steps_at_a_time_equal_single_steps(gpu, method, dims):
+    """Without solid cells a call of several steps takes them two at a time: same bits as one step per call, at
+    whole and partial tiles, odd widths, chunk ends, and extents that wrap onto themselves."""
+    fields = init_fields(*dims, seed=23)
+    om = 1.3 if method == METHOD_HYBRID else None
+    one = run_gpu(method, dims, 0.56, fields, None, 12, force=(1e-5, 2e-6, -1e-6), omega_s=om, chunks=[1] * 12, stats=True)
+    for chunks in ([12], [1, 4, 7], [2, 10], [6, 6]):
+        many = run_gpu(method, dims, 0.56, fields, None, 12, force=(1e-5, 2e-6, -1e-6), omega_s=om, chunks=chunks, stats=True)
+        np.testing.assert_array_equal(many["state"], one["state"])
+        for a, b in zip(many["macros"], one["macros"]):
+            np.testing.assert_array_equal(a, b)
+        assert many["stats"] == one["stats"]
+
+
 def test_hybrid_equals_legacy_by_default(gpu):
     """omega_s = omega_h makes the two collision forms the same arithmetic (hybrid.cu:264-267)."""
     dims = (16, 12, 10)
