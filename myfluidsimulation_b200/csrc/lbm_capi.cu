@@ -404,7 +404,7 @@ int lbm_create(const lbm_domain* dom, const lbm_options* opts, lbm_solver** out)
         s->home_zchunk = std::min(zc, dom->nz);
     }
     // the z-marching odd step's grid (solvers without a mask)
-    const int64_t odd_blocks = lbm::aa_odd_blocks(dom->nx, dom->ny, dom->nz, false, o.storage, s->cfg_odd.threads);
+    const int64_t odd_blocks = lbm::aa_odd_blocks(dom->nx, dom->ny, dom->nz, o.storage, s->cfg_odd.threads);
     s->max_blocks = (int)std::max<int64_t>({s->cfg_even.blocks, s->cfg_odd.blocks, odd_blocks,
                                             lbm::home_num_blocks(dom->nx, dom->ny, dom->nz, s->home_zchunk), 1});
     auto dmalloc = [&](void** p, size_t b) { return cudaMalloc(p, b) == cudaSuccess; };

@@ -32,7 +32,8 @@ struct AAParams {
     // ghost copies of the neighbouring slabs' boundary planes
     int64_t first, cells;
     uint32_t salt_base;      // F16/BF16 stochastic rounding: index of cell 0 in the whole grid
-    int zrun;                // odd step: planes per block (set by launch_aa_step)
+    int zrun;                // odd step: planes per block, cells of a row per block and
+    int bx, by;              // rows per block (set by launch_aa_step)
 };
 
 // Parameters of one HOME step (moment-only, two buffers).
@@ -66,10 +67,9 @@ struct LaunchCfg {
 // AA steps.  parity 0: natural layout in (the even, purely local step);
 // parity 1: the odd step (gathers from and scatters to neighbours).
 cudaError_t launch_aa_step(const AAParams& p, int storage, int parity, LaunchCfg cfg, cudaStream_t s);
-// the odd step's grid: blocks of `threads` cells of one row, each over a run of
-// aa_odd_zrun planes; one statistics partial per block
-int aa_odd_zrun(int nx, int ny, int64_t planes, bool mask, int storage, int threads);
-int64_t aa_odd_blocks(int nx, int ny, int64_t planes, bool mask, int storage, int threads);
+// the z-marching odd step's grid: blocks of at most `threads` cells of one or more
+// rows, each over a run of planes; one statistics partial per block
+int64_t aa_odd_blocks(int nx, int ny, int64_t planes, int storage, int threads);
 // blocks of one odd-step launch: the z-marching grid without a mask; with one,
 // cfg.blocks rounded down to a multiple of the row segments (a 2-D grid of
 // rows x segments)
