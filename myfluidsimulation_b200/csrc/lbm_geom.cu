@@ -7,10 +7,11 @@
 //     every float operation is spelled with an explicit rounding intrinsic
 //     (__fadd_rn, __fmul_rn, ...), so nvcc cannot contract it into an FMA and
 //     each result equals the reference's uncontracted x86-64 float result;
-//   * the exterior flood fill is a reachability fixed point, computed by
-//     rounds of six directional line sweeps (+-x, +-y, +-z) until a round
-//     changes nothing; the reachable set is unique, so the mask is identical
-//     to the BFS result whatever the visiting order;
+//   * the grid is held as one bit per cell, 32 cells along x to a word;
+//   * the exterior flood fill is a reachability fixed point: one block per (x, y)
+//     plane floods its plane to the end in shared memory, then one per (x, z)
+//     plane, until a round changes nothing; the reachable set is unique, so the
+//     mask is identical to the BFS result whatever the visiting order;
 //   * the optional refine^3 coverage downsample (voxelize.cpp:187-226) is one
 //     thread per coarse cell.
 #include "lbm_common.cuh"
@@ -95,7 +96,7 @@ __global__ void fit_kernel(const float* __restrict__ in, float* __restrict__ out
 
 // voxelize.cpp:115-149: one warp per triangle
 __global__ void surface_kernel(const float* __restrict__ vt, int64_t ntri, int nx, int ny, int nz,
-                               uint8_t* __restrict__ surf) {
+                               int wx, uint32_t* __restrict__ surf) {
     const int lane = threadIdx.x & 31;
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
     const float h[3] = {__fdiv_rn(0.5f, (float)nx), __fdiv_rn(0.5f, (float)ny), __fdiv_rn(0.5f, (float)nz)};
@@ -122,58 +123,149 @@ __global__ void surface_kernel(const float* __restrict__ vt, int64_t ntri, int n
             const float cc[3] = {__fdiv_rn(__fadd_rn((float)x, 0.5f), (float)nx),
                                  __fdiv_rn(__fadd_rn((float)y, 0.5f), (float)ny),
                                  __fdiv_rn(__fadd_rn((float)z, 0.5f), (float)nz)};
-            if (tri_box(cc, h, v0, v1, v2)) surf[((int64_t)z * ny + y) * nx + x] = 1;
+            if (tri_box(cc, h, v0, v1, v2)) atomicOr(surf + ((int64_t)z * ny + y) * wx + (x >> 5), 1u << (x & 31));
         }
     }
 }
 
-// seeds: non-surface cells on the six faces (voxelize.cpp:160-163)
-__global__ void seed_kernel(const uint8_t* __restrict__ surf, uint8_t* __restrict__ vis, int nx, int ny, int nz) {
-    const int64_t N = (int64_t)nx * ny * nz;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
-        const int x = (int)(i % nx);
-        const int64_t row = i / nx;
-        const int y = (int)(row % ny), z = (int)(row / ny);
-        const bool face = x == 0 || x == nx - 1 || y == 0 || y == ny - 1 || z == 0 || z == nz - 1;
-        vis[i] = (face && !surf[i]) ? 1 : 0;
-    }
-}
-
-// One directional sweep: each thread walks one line of the grid along `axis`
-// in direction `dir`, carrying "reached" across non-surface cells.
-__global__ void sweep_kernel(const uint8_t* __restrict__ surf, uint8_t* __restrict__ vis, int nx, int ny, int nz,
-                             int axis, int dir, int* changed) {
-    const int n[3] = {nx, ny, nz};
-    const int64_t stride[3] = {1, nx, (int64_t)nx * ny};
-    const int a1 = axis == 0 ? 1 : 0, a2 = axis == 2 ? 1 : 2;
-    const int64_t lines = (int64_t)n[a1] * n[a2];
-    int any = 0;
-    for (int64_t l = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; l < lines; l += (int64_t)gridDim.x * blockDim.x) {
-        const int i1 = (int)(l % n[a1]), i2 = (int)(l / n[a1]);
-        const int64_t base = i1 * stride[a1] + i2 * stride[a2];
-        bool carry = false;
-        for (int s = 0; s < n[axis]; ++s) {
-            const int c = dir > 0 ? s : n[axis] - 1 - s;
-            const int64_t id = base + c * stride[axis];
-            if (surf[id]) { carry = false; continue; }
-            if (vis[id]) { carry = true; continue; }
-            if (carry) { vis[id] = 1; any = 1; }
+// One plane of the flood fill: `rows` rows of `wx` words, open cells O, reached
+// cells R (a subset of O), `pitch` words from row to row.  Sweeps along x and across the rows
+// alternate until nothing changes.
+//   x: a carry ripples through a run of ones, so (O + R) ^ O marks the run from a
+//      seed upward; one thread per row, the carry going from word to word, then
+//      the same on reversed bits.
+//   rows: 32 cells at a time; every word column is cut into segments, one thread
+//      per segment finds what leaves it (from inside, and with everything entering),
+//      the segments are chained, and each is swept once more with what enters it.
+__device__ bool flood_plane(const uint32_t* __restrict__ O, uint32_t* R, int rows, int wx, int64_t pitch,
+                            uint32_t* seg) {
+    const int T = (int)blockDim.x, tid = (int)threadIdx.x;
+    const int nseg = max(1, min(T / wx, rows)), len = (rows + nseg - 1) / nseg;
+    uint32_t *sa = seg, *sb = seg + T;
+    bool ever = false;
+    for (;;) {
+        bool any = false;
+        for (int y = tid; y < rows; y += T) {
+            const uint32_t* o = O + (int64_t)y * pitch;
+            uint32_t* r = R + (int64_t)y * pitch;
+            uint32_t in = 0;      // the last cell of the word before is reached
+            for (int w = 0; w < wx; ++w) {
+                const uint32_t ow = o[w], rw = r[w];
+                const uint32_t sd = rw | (in & ow);
+                const uint32_t n = sd | (ow & (ow ^ (ow + sd)));
+                if (n != rw) { r[w] = n; any = true; }
+                in = n >> 31;
+            }
+            in = 0;
+            for (int w = wx - 1; w >= 0; --w) {
+                const uint32_t rw = r[w], ow = __brev(o[w]), rv = __brev(rw);
+                const uint32_t sd = rv | (in & ow);
+                const uint32_t n = sd | (ow & (ow ^ (ow + sd)));
+                if (n != rv) { r[w] = __brev(n); any = true; }
+                in = n >> 31;
+            }
         }
+        __syncthreads();
+        for (int c0 = 0; c0 < wx; c0 += T) {          // word columns in groups of at most T
+            const int cols = min(wx - c0, T);
+            for (int dir = 0; dir < 2; ++dir) {
+                const int w = c0 + tid % cols, k = tid / cols;
+                const int y0 = k * len, y1 = min(rows, y0 + len);
+                const bool on = k < nseg && y0 < rows;
+                auto row = [&](int i) { return (int64_t)(dir ? rows - 1 - i : i) * pitch + w; };
+                if (on) {
+                    uint32_t out = 0, through = 0xffffffffu;
+                    for (int i = y0; i < y1; ++i) {
+                        const uint32_t o = O[row(i)];
+                        out = R[row(i)] | (out & o);
+                        through &= o;
+                    }
+                    sa[tid] = out;
+                    sb[tid] = through;
+                }
+                __syncthreads();
+                if (on) {
+                    uint32_t c = 0;
+                    for (int j = 0; j < k; ++j) c = sa[j * cols + tid % cols] | (c & sb[j * cols + tid % cols]);
+                    for (int i = y0; i < y1; ++i) {
+                        const uint32_t o = O[row(i)], r = R[row(i)];
+                        c = r | (c & o);
+                        if (c != r) { R[row(i)] = c; any = true; }
+                    }
+                }
+                __syncthreads();
+            }
+        }
+        if (!__syncthreads_or(any)) return ever;
+        ever = true;
     }
-    if (any) atomicOr(changed, 1);
 }
 
-__global__ void solid_kernel(const uint8_t* __restrict__ surf, const uint8_t* __restrict__ vis,
-                             uint8_t* __restrict__ out, int64_t N) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x)
-        out[i] = (surf[i] || !vis[i]) ? 1 : 0;
+// Flood of one (x, y) plane per block (AXIS 2) or one (x, z) plane (AXIS 1).
+// first: the exterior starts from the open cells on the six faces.  A round whose
+// predecessor changed nothing (changed[round - 1] == 0) has nothing to do.  SHARED:
+// the plane's words fit in shared memory; otherwise it is flooded where it lies.
+template <int AXIS, bool SHARED>
+__global__ void __launch_bounds__(512) flood_kernel(const uint32_t* __restrict__ surf, uint32_t* vis, int nx, int ny,
+                                                    int nz, int wx, int first, int round, int* changed) {
+    extern __shared__ uint32_t buf[];
+    __shared__ uint32_t seg[2 * 512];
+    if (round > 0 && changed[round - 1] == 0) return;
+    const int rows = AXIS == 2 ? ny : nz;
+    const int64_t pitch = AXIS == 2 ? wx : (int64_t)ny * wx;
+    const int64_t base = AXIS == 2 ? (int64_t)blockIdx.x * ny * wx : (int64_t)blockIdx.x * wx;
+    const uint32_t last = nx % 32 ? (1u << (nx % 32)) - 1u : 0xffffffffu;
+    uint32_t* O = buf;                          // (not SHARED: vis + the second half of the buffer)
+    uint32_t* R = SHARED ? buf + rows * wx : vis + base;
+    const bool face = AXIS == 2 && (blockIdx.x == 0 || blockIdx.x == (unsigned)nz - 1);
+    bool seeded = false;
+    for (int i = threadIdx.x; i < rows * wx; i += blockDim.x) {
+        const int y = i / wx, w = i - y * wx;
+        const int64_t g = base + (int64_t)y * pitch + w;
+        const uint32_t o = ~surf[g] & (w == wx - 1 ? last : 0xffffffffu);
+        uint32_t r;
+        if (first) {
+            uint32_t m = face || y == 0 || y == ny - 1 ? 0xffffffffu : 0u;
+            if (w == 0) m |= 1u;
+            if (w == wx - 1) m |= 1u << ((nx - 1) & 31);
+            r = o & m;
+            seeded = seeded || r != 0;
+        } else {
+            r = vis[g];
+        }
+        if (SHARED) { O[i] = o; R[i] = r; }
+        else if (first) vis[g] = r;
+    }
+    bool ch;
+    if constexpr (SHARED) {
+        __syncthreads();
+        ch = flood_plane(O, R, rows, wx, wx, seg);
+        if (ch || first)
+            for (int i = threadIdx.x; i < rows * wx; i += blockDim.x) {
+                const int y = i / wx, w = i - y * wx;
+                vis[base + (int64_t)y * pitch + w] = R[i];
+            }
+    } else {
+        __syncthreads();
+        ch = flood_plane(vis + (int64_t)nz * ny * wx + base, vis + base, rows, wx, pitch, seg);   // open cells: second half
+    }
+    if (__syncthreads_or(ch || seeded) && threadIdx.x == 0) changed[round] = 1;
 }
 
-// voxelize.cpp:187-226
-__global__ void downsample_kernel(const uint8_t* __restrict__ fine, int r, int nx, int ny, int nz, float thr,
-                                  uint8_t* __restrict__ out) {
+// the open cells of a grid whose planes do not fit in shared memory
+__global__ void open_kernel(const uint32_t* __restrict__ surf, uint32_t* __restrict__ open, int64_t words, int wx,
+                            uint32_t last) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < words; i += (int64_t)gridDim.x * blockDim.x)
+        open[i] = ~surf[i] & (i % wx == wx - 1 ? last : 0xffffffffu);
+}
+
+// Solid = surface or not reached; with refinement r the coverage of r^3 fine cells
+// against thr (voxelize.cpp:187-226).  One thread per coarse cell, whose r cells of
+// a fine row lie in one or two words (r <= 32) or are counted word by word.
+__global__ void mask_kernel(const uint32_t* __restrict__ surf, const uint32_t* __restrict__ vis, int r, int nx, int ny,
+                            int nz, int wx, float thr, uint8_t* __restrict__ out) {
     const int64_t N = (int64_t)nx * ny * nz;
-    const int64_t fx = (int64_t)nx * r, fy = (int64_t)ny * r;
+    const int64_t fy = (int64_t)ny * r;
     const int r3 = r * r * r;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
         const int x = (int)(i % nx);
@@ -182,11 +274,21 @@ __global__ void downsample_kernel(const uint8_t* __restrict__ fine, int r, int n
         int cnt = 0;
         for (int dz = 0; dz < r; ++dz)
             for (int dy = 0; dy < r; ++dy) {
-                const int64_t b = ((int64_t)z * r + dz) * fy * fx + ((int64_t)y * r + dy) * fx + (int64_t)x * r;
-                for (int dx = 0; dx < r; ++dx) cnt += fine[b + dx];
+                const int64_t b = (((int64_t)z * r + dz) * fy + (int64_t)y * r + dy) * wx;
+                int64_t x0 = (int64_t)x * r, left = r;
+                while (left > 0) {
+                    const int bit = (int)(x0 & 31), take = (int)min((int64_t)(32 - bit), left);
+                    const uint32_t m = (take == 32 ? 0xffffffffu : ((1u << take) - 1u)) << bit;
+                    cnt += __popc((surf[b + (x0 >> 5)] | ~vis[b + (x0 >> 5)]) & m);
+                    x0 += take;
+                    left -= take;
+                }
             }
-        const float cov = __fdiv_rn((float)cnt, (float)r3);
-        out[i] = (cov > 0.0f && cov >= thr) ? 1 : 0;
+        if (r == 1) out[i] = (uint8_t)cnt;
+        else {
+            const float cov = __fdiv_rn((float)cnt, (float)r3);
+            out[i] = (cov > 0.0f && cov >= thr) ? 1 : 0;
+        }
     }
 }
 
@@ -208,53 +310,64 @@ cudaError_t launch_voxelize(const float* d_tris, int64_t ntri, const float* bb, 
     }
     const int fx = nx * refine, fy = ny * refine, fz = nz * refine;
     const int64_t NF = (int64_t)fx * fy * fz;
+    const int wx = (fx + 31) / 32;
+    const int64_t words = NF / fx * wx;
+    const size_t sm2 = sizeof(uint32_t) * 2 * (size_t)fy * wx, sm1 = sizeof(uint32_t) * 2 * (size_t)fz * wx;
+    constexpr size_t kShared = 200 * 1024;     // beyond it a plane is flooded in global memory
+    const bool shared = sm2 <= kShared && sm1 <= kShared;
+    constexpr int kRounds = 16;                // rounds queued between two looks at the result
     float* vt = nullptr;
-    uint8_t *surf = nullptr, *vis = nullptr, *fine = nullptr;
+    uint32_t *surf = nullptr, *vis = nullptr;
     int* changed = nullptr;
     cudaError_t e = cudaSuccess;
 #define VX_CK(x) do { e = (x); if (e != cudaSuccess) goto done; } while (0)
     VX_CK(cudaMallocAsync(&vt, sizeof(float) * 9 * (size_t)(ntri > 0 ? ntri : 1), s));
-    VX_CK(cudaMallocAsync(&surf, (size_t)NF, s));
-    VX_CK(cudaMallocAsync(&vis, (size_t)NF, s));
-    VX_CK(cudaMallocAsync(&changed, sizeof(int), s));
-    if (refine > 1) VX_CK(cudaMallocAsync(&fine, (size_t)NF, s));
-    VX_CK(cudaMemsetAsync(surf, 0, (size_t)NF, s));
+    VX_CK(cudaMallocAsync(&surf, sizeof(uint32_t) * (size_t)words, s));
+    VX_CK(cudaMallocAsync(&vis, sizeof(uint32_t) * (size_t)words * (shared ? 1 : 2), s));
+    VX_CK(cudaMallocAsync(&changed, sizeof(int) * kRounds, s));
+    VX_CK(cudaMemsetAsync(surf, 0, sizeof(uint32_t) * (size_t)words, s));
     if (ntri > 0) {
         fit_kernel<<<num_sms() * 4, 256, 0, s>>>(d_tris, vt, ntri * 9, sf, tr[0], tr[1], tr[2]);
         const int64_t blocks = (ntri + 7) / 8;   // 8 warps per block
-        surface_kernel<<<(int)(blocks < 65535 ? blocks : 65535), 256, 0, s>>>(vt, ntri, fx, fy, fz, surf);
+        surface_kernel<<<(int)(blocks < 65535 ? blocks : 65535), 256, 0, s>>>(vt, ntri, fx, fy, fz, wx, surf);
         VX_CK(cudaGetLastError());
     }
-    seed_kernel<<<num_sms() * 8, 256, 0, s>>>(surf, vis, fx, fy, fz);
-    VX_CK(cudaGetLastError());
-    for (int round = 0; round < 1000000; ++round) {
-        VX_CK(cudaMemsetAsync(changed, 0, sizeof(int), s));
-        for (int axis = 0; axis < 3; ++axis)
-            for (int dir = -1; dir <= 1; dir += 2) {
-                const int64_t lines = (axis == 0) ? (int64_t)fy * fz : (axis == 1 ? (int64_t)fx * fz : (int64_t)fx * fy);
-                const int64_t b = (lines + 127) / 128;
-                sweep_kernel<<<(int)(b < 65535 ? b : 65535), 128, 0, s>>>(surf, vis, fx, fy, fz, axis, dir, changed);
-            }
-        VX_CK(cudaGetLastError());
-        int h = 0;
-        VX_CK(cudaMemcpyAsync(&h, changed, sizeof(int), cudaMemcpyDeviceToHost, s));
-        VX_CK(cudaStreamSynchronize(s));
-        if (!h) break;
-    }
-    if (refine == 1) {
-        solid_kernel<<<num_sms() * 8, 256, 0, s>>>(surf, vis, d_mask, NF);
+    if (shared) {
+        VX_CK(cudaFuncSetAttribute((const void*)flood_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kShared));
+        VX_CK(cudaFuncSetAttribute((const void*)flood_kernel<1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kShared));
     } else {
-        solid_kernel<<<num_sms() * 8, 256, 0, s>>>(surf, vis, fine, NF);
-        const float t = fmaxf(0.0f, fminf(1.0f, thr));
-        downsample_kernel<<<num_sms() * 8, 256, 0, s>>>(fine, refine, nx, ny, nz, t, d_mask);
+        const uint32_t last = fx % 32 ? (1u << (fx % 32)) - 1u : 0xffffffffu;
+        open_kernel<<<num_sms() * 8, 256, 0, s>>>(surf, vis + words, words, wx, last);
+        VX_CK(cudaGetLastError());
     }
+    for (int pass = 0;; ++pass) {
+        // (the first batch: most obstacles are done after one round, which the second one confirms)
+        const int n = pass == 0 ? 3 : kRounds;
+        int h[kRounds];
+        VX_CK(cudaMemsetAsync(changed, 0, sizeof(int) * kRounds, s));
+        for (int k = 0; k < n; ++k) {
+            const int first = pass == 0 && k == 0;
+            if (shared) {
+                flood_kernel<2, true><<<fz, 512, sm2, s>>>(surf, vis, fx, fy, fz, wx, first, k, changed);
+                flood_kernel<1, true><<<fy, 512, sm1, s>>>(surf, vis, fx, fy, fz, wx, 0, k, changed);
+            } else {
+                flood_kernel<2, false><<<fz, 512, 0, s>>>(surf, vis, fx, fy, fz, wx, first, k, changed);
+                flood_kernel<1, false><<<fy, 512, 0, s>>>(surf, vis, fx, fy, fz, wx, 0, k, changed);
+            }
+            VX_CK(cudaGetLastError());
+        }
+        VX_CK(cudaMemcpyAsync(h, changed, sizeof(int) * kRounds, cudaMemcpyDeviceToHost, s));
+        VX_CK(cudaStreamSynchronize(s));
+        if (!h[n - 1]) break;
+    }
+    mask_kernel<<<num_sms() * 8, 256, 0, s>>>(surf, vis, refine, nx, ny, nz, wx,
+                                              fmaxf(0.0f, fminf(1.0f, thr)), d_mask);
     VX_CK(cudaGetLastError());
 done:
 #undef VX_CK
     if (vt) cudaFreeAsync(vt, s);
     if (surf) cudaFreeAsync(surf, s);
     if (vis) cudaFreeAsync(vis, s);
-    if (fine) cudaFreeAsync(fine, s);
     if (changed) cudaFreeAsync(changed, s);
     return e;
 }

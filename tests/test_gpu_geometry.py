@@ -82,3 +82,20 @@ def test_gpu_stl_loader_matches(gpu, oracle, tmp_path):
         t, bb = oracle.load_stl(p)
         np.testing.assert_array_equal(m.tris, t)
         np.testing.assert_array_equal(np.concatenate([m.bbmin, m.bbmax]), bb)
+
+
+@pytest.mark.parametrize("dims,refine", [((31, 33, 5), 1), ((32, 7, 64), 1), ((65, 18, 17), 2), ((11, 40, 23), 3), ((1, 3, 40), 1),
+                                         ((700, 660, 2), 2)])      # planes too large for shared memory
+def test_voxelizer_flood_fill_of_shells_vs_oracle(gpu, oracle, dims, refine):
+    """A shell with a hole leads into a cavity that only winding paths reach, next to a closed one: partial last
+    words, single words, several words per row, refined grids."""
+    tris = W.icosphere(2)
+    big = tris * 1.0
+    big = big[np.abs(big.mean(1) - np.array([0.0, 0.0, 1.0])).max(1) > 0.35]          # open at +z
+    inner = tris * 0.45
+    shell = np.concatenate([big, inner, tris * 0.3 + np.array([0.0, 0.75, 0.0])]).astype(np.float32)
+    mesh = G.mesh_from_triangles(shell)
+    p = G.VoxelParams(*dims, 0.9, (0.5, 0.5, 0.5), refine, 0.5)
+    got = G.voxelize_mesh_to_mask(mesh, p)
+    want = oracle.voxelize(shell, mesh_bbox(shell), dims, 0.9, (0.5, 0.5, 0.5), refine, 0.5)
+    np.testing.assert_array_equal(got, want)
