@@ -2,6 +2,8 @@
 // flag/link words built from the solid mask, the B0 band, the final pass of
 // the FP64 statistics, and the reference's free device helpers
 // (reinit_equilibrium_from_macro, launch_speed, make_rho_gauss/slab).
+#include <mutex>
+
 #include "lbm_common.cuh"
 #include "lbm_internal.h"
 
@@ -16,6 +18,32 @@ int num_sms() {
         if (n <= 0) n = 148;
     }
     return n;
+}
+
+cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s) {
+    constexpr int kDevices = 64;
+    static std::mutex mu;
+    static cudaMemPool_t pools[kDevices] = {};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev >= kDevices) return cudaMallocAsync(p, bytes, s);
+    cudaMemPool_t pool = nullptr;
+    {
+        std::lock_guard<std::mutex> g(mu);
+        if (!pools[dev]) {
+            cudaMemPoolProps props{};
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = dev;
+            e = cudaMemPoolCreate(&pools[dev], &props);
+            if (e != cudaSuccess) { pools[dev] = nullptr; return e; }
+            uint64_t keep = kScratchKept;
+            cudaMemPoolSetAttribute(pools[dev], cudaMemPoolAttrReleaseThreshold, &keep);
+        }
+        pool = pools[dev];
+    }
+    return cudaMallocFromPoolAsync(p, bytes, pool, s);
 }
 
 namespace {

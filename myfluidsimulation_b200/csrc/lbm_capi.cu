@@ -1132,8 +1132,8 @@ int lbm_voxelize(const float* tris, int64_t ntri, const float* bb_in, const lbm_
     CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
     float* d_tris = nullptr;
     uint8_t* d_mask = nullptr;
-    cudaError_t e = cudaMallocAsync((void**)&d_tris, sizeof(float) * 9 * (size_t)(ntri > 0 ? ntri : 1), st);
-    if (e == cudaSuccess) e = cudaMallocAsync((void**)&d_mask, (size_t)N, st);
+    cudaError_t e = lbm::scratch_alloc((void**)&d_tris, sizeof(float) * 9 * (size_t)(ntri > 0 ? ntri : 1), st);
+    if (e == cudaSuccess) e = lbm::scratch_alloc((void**)&d_mask, (size_t)N, st);
     if (e == cudaSuccess && ntri > 0)
         e = cudaMemcpyAsync(d_tris, tris, sizeof(float) * 9 * (size_t)ntri, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess)

@@ -321,10 +321,10 @@ cudaError_t launch_voxelize(const float* d_tris, int64_t ntri, const float* bb, 
     int* changed = nullptr;
     cudaError_t e = cudaSuccess;
 #define VX_CK(x) do { e = (x); if (e != cudaSuccess) goto done; } while (0)
-    VX_CK(cudaMallocAsync(&vt, sizeof(float) * 9 * (size_t)(ntri > 0 ? ntri : 1), s));
-    VX_CK(cudaMallocAsync(&surf, sizeof(uint32_t) * (size_t)words, s));
-    VX_CK(cudaMallocAsync(&vis, sizeof(uint32_t) * (size_t)words * (shared ? 1 : 2), s));
-    VX_CK(cudaMallocAsync(&changed, sizeof(int) * kRounds, s));
+    VX_CK(scratch_alloc((void**)&vt, sizeof(float) * 9 * (size_t)(ntri > 0 ? ntri : 1), s));
+    VX_CK(scratch_alloc((void**)&surf, sizeof(uint32_t) * (size_t)words, s));
+    VX_CK(scratch_alloc((void**)&vis, sizeof(uint32_t) * (size_t)words * (shared ? 1 : 2), s));
+    VX_CK(scratch_alloc((void**)&changed, sizeof(int) * kRounds, s));
     VX_CK(cudaMemsetAsync(surf, 0, sizeof(uint32_t) * (size_t)words, s));
     if (ntri > 0) {
         fit_kernel<<<num_sms() * 4, 256, 0, s>>>(d_tris, vt, ntri * 9, sf, tr[0], tr[1], tr[2]);

@@ -8,13 +8,13 @@
 // host and the device builds give the same text; a CPU test checks it against
 // the C library's printf.
 //
-// A field of N cells becomes N lines ("v\n", "|u|\n" or "u v w\n").  Two
-// kernels: vtk_count formats every line of a block of 256 and stores the
-// block's byte count; vtk_scan turns the counts into offsets (one block);
-// vtk_emit formats again, scans the line lengths inside the block and stores
-// the block's text at its offset.  Formatting costs a few hundred integer
-// operations per value, far below the cost of moving the text to the host, so
-// formatting twice beats storing per-line lengths.
+// A field of N cells becomes N lines ("v\n", "|u|\n" or "u v w\n").  One kernel,
+// vtk_emit: a block takes 256 lines, finds each value's six digits and exponent
+// once (g6_parse), which give the line lengths, gets its place in the text from
+// the blocks before it by looking back over their published lengths, writes the
+// characters (g6_put) to shared memory where they belong, and stores the block's
+// text with 4-byte words.  Blocks number themselves in the order they start, so a
+// block only ever waits for blocks that are already running.
 //
 // lbm_vtk_writer runs the whole snapshot asynchronously: the kernels are
 // queued on the caller's stream (ordered after the step that produced the
@@ -143,89 +143,138 @@ HD uint32_t scaled_floor(uint32_t m, int e, int s, int& half) {
     return n;
 }
 
-// Bytes of printf("%g", (double)v) into out (at most 12); returns the length.
-HD int fmt_g6(float v, char* out) {
+// 10^k for 0 <= k <= 22, all exact doubles
+#define G6_POW10                                                                                                   \
+    {1e0, 1e1, 1e2, 1e3, 1e4, 1e5, 1e6, 1e7, 1e8, 1e9, 1e10, 1e11, 1e12, 1e13, 1e14, 1e15, 1e16, 1e17, 1e18, 1e19, \
+     1e20, 1e21, 1e22}
+
+// A value as printf("%g") shows it: six digits n (100000 .. 999999), decimal
+// exponent x, sign, and kind 0 (a number), 1 (zero), 2 (inf), 3 (nan).
+struct G6 {
+    uint32_t n;
+    int8_t x;
+    uint8_t neg, kind;
+    uint8_t last;      // index of the last digit kept (trailing zeros are dropped)
+};
+
+// the digits by exact integer comparison: values next to a rounding or digit boundary
+HD void g6_exact(uint32_t m, int e, int& X, uint32_t& n, int& half) {
+    for (int it = 0; it < 4; ++it) {
+        n = scaled_floor(m, e, 5 - X, half);
+        if (n >= 1000000u) { ++X; continue; }
+        if (n < 100000u) { --X; continue; }
+        break;
+    }
+}
+
+// p10: the powers of ten (shared memory on the device)
+HD G6 g6_parse(float v, const double* p10) {
+    G6 g{};
     uint32_t bits;
     memcpy(&bits, &v, 4);
-    const bool neg = bits >> 31;
+    g.neg = (uint8_t)(bits >> 31);
     const uint32_t E = (bits >> 23) & 0xffu, F = bits & 0x7fffffu;
-    int len = 0;
-    if (neg) out[len++] = '-';
-    if (E == 0xffu) {
-        const char* s = F ? "nan" : "inf";
-        out[len++] = s[0]; out[len++] = s[1]; out[len++] = s[2];
-        return len;
-    }
-    if (E == 0 && F == 0) { out[len++] = '0'; return len; }
+    if (E == 0xffu) { g.kind = F ? 3 : 2; return g; }
+    if (E == 0 && F == 0) { g.kind = 1; return g; }
     const uint32_t m = E ? (F | 0x800000u) : F;
     const int e = (E ? (int)E : 1) - 150;
     // decimal exponent: floor(log10 v), from the bit length, then corrected
-    int b = 0;
-    for (uint32_t x = m; x; x >>= 1) ++b;
+#ifdef __CUDA_ARCH__
+    const int b = 32 - __clz((int)m);
+#else
+    const int b = 32 - __builtin_clz(m);
+#endif
     const int l2 = b - 1 + e;                                  // floor(log2 v)
     int X = (l2 >= 0) ? (l2 * 78913) >> 18 : -((-l2 * 78913 + 262143) >> 18);   // ~ l2 * log10(2)
     uint32_t n = 0;
     int half = 0;
     // fast path: y = v 10^k in double with one correctly rounded operation
     // (10^|k| is exact for |k| <= 22), so |y - exact| <= 2^-33 for y < 2^20;
-    // taken only when floor(y) and the side of one half are certain, else the
-    // exact path below decides
+    // taken only when floor(y) and the side of one half are certain (y is exact,
+    // or far enough from both), else the exact path below decides
+    const double x = (double)(bits >> 31 ? -v : v);
     bool done = false;
     for (int it = 0; it < 3; ++it) {
         const int k = 5 - X;
         if (k < -22 || k > 22) break;
-        double p = 1.0, sq = 10.0;
-        for (int a = k < 0 ? -k : k; a; a >>= 1, sq *= sq)
-            if (a & 1) p *= sq;
-        const double x = ldexp((double)m, e);
+        const double p = p10[k < 0 ? -k : k];
         const double y = k >= 0 ? x * p : x / p;
-        const double fl = floor(y);
-        if (fl >= 1000000.0) { ++X; continue; }
-        if (fl < 100000.0) { --X; continue; }
-        const double fr = y - fl, tol = 0x1p-30;
-        if (fr < tol || fr > 1.0 - tol || fabs(fr - 0.5) < tol) break;
-        n = (uint32_t)fl;
-        half = fr > 0.5 ? 1 : -1;
+        if (y >= 1000000.0) { ++X; continue; }
+        if (y < 100000.0) { --X; continue; }
+        const uint32_t fl = (uint32_t)y;
+        const double fr = y - (double)fl, tol = 0x1p-30;
+        const bool exact = k >= 0 && fma(x, p, -y) == 0.0;
+        if (!exact && (fr < tol || fr > 1.0 - tol || fabs(fr - 0.5) < tol)) break;
+        n = fl;
+        half = fr > 0.5 ? 1 : (fr < 0.5 ? -1 : 0);
         done = true;
         break;
     }
-    for (int it = 0; !done && it < 4; ++it) {
-        n = scaled_floor(m, e, 5 - X, half);
-        if (n >= 1000000u) { ++X; continue; }
-        if (n < 100000u) { --X; continue; }
-        break;
-    }
+    if (!done) g6_exact(m, e, X, n, half);
     if (half > 0 || (half == 0 && (n & 1u))) {
         if (++n == 1000000u) { n = 100000u; ++X; }
     }
-    char d[6];
-    for (int i = 5; i >= 0; --i) { d[i] = (char)('0' + n % 10u); n /= 10u; }
-    int last = 5;                                              // last significant digit kept
-    while (last > 0 && d[last] == '0') --last;
-    if (X < -4 || X >= 6) {
-        out[len++] = d[0];
-        if (last > 0) {
-            out[len++] = '.';
-            for (int i = 1; i <= last; ++i) out[len++] = d[i];
-        }
-        out[len++] = 'e';
-        out[len++] = X < 0 ? '-' : '+';
-        const int a = X < 0 ? -X : X;
-        out[len++] = (char)('0' + a / 10);
-        out[len++] = (char)('0' + a % 10);
-    } else if (X >= 0) {
-        for (int i = 0; i <= X; ++i) out[len++] = d[i];
-        if (last > X) {
-            out[len++] = '.';
-            for (int i = X + 1; i <= last; ++i) out[len++] = d[i];
-        }
-    } else {
-        out[len++] = '0';
-        out[len++] = '.';
-        for (int i = 0; i < -X - 1; ++i) out[len++] = '0';
-        for (int i = 0; i <= last; ++i) out[len++] = d[i];
+    g.n = n;
+    g.x = (int8_t)X;
+    // trailing zeros
+    uint32_t r = n;
+    int last = 5;
+    while (last > 0 && r % 10u == 0u) { r /= 10u; --last; }
+    g.last = (uint8_t)last;
+    return g;
+}
+
+// number of characters of g
+HD int g6_len(const G6& g) {
+    const int neg = g.neg;
+    if (g.kind) return neg + (g.kind == 1 ? 1 : 3);
+    const int X = g.x, last = g.last;
+    if (X < -4 || X >= 6) return neg + 1 + (last > 0 ? last + 1 : 0) + 4;
+    if (X >= 0) return neg + X + 1 + (last > X ? 1 + last - X : 0);
+    return neg + 2 + (-X - 1) + last + 1;
+}
+
+// the characters of g into out (at most 12); returns their number
+HD int g6_put(const G6& g, char* out) {
+    char* o = out;
+    if (g.neg) *o++ = '-';
+    if (g.kind) {
+        if (g.kind == 1) { *o++ = '0'; return (int)(o - out); }
+        const bool nan = g.kind == 3;
+        *o++ = nan ? 'n' : 'i'; *o++ = nan ? 'a' : 'n'; *o++ = nan ? 'n' : 'f';
+        return (int)(o - out);
     }
-    return len;
+    const int X = g.x, last = g.last;
+    // where the point goes: behind digit `point` (-1: in front of all, after "0." and zeros)
+    const bool ex = X < -4 || X >= 6;
+    const int point = ex ? 0 : X;
+    if (point < 0) {
+        *o++ = '0';
+        *o++ = '.';
+        for (int i = 0; i < -X - 1; ++i) *o++ = '0';
+    }
+    uint32_t r = g.n, p = 100000u;
+    for (int i = 0; i < 6; ++i) {
+        const uint32_t d = r / p;
+        r -= d * p;
+        p /= 10u;
+        if (i <= last || i <= point) *o++ = (char)('0' + d);
+        if (i == point && last > point) *o++ = '.';
+    }
+    if (ex) {
+        *o++ = 'e';
+        *o++ = X < 0 ? '-' : '+';
+        const int a = X < 0 ? -X : X;
+        *o++ = (char)('0' + a / 10);
+        *o++ = (char)('0' + a % 10);
+    }
+    return (int)(o - out);
+}
+
+// Bytes of printf("%g", (double)v) into out (at most 12); returns the length.
+inline int fmt_g6(float v, char* out) {
+    static const double p10[23] = G6_POW10;
+    return g6_put(g6_parse(v, p10), out);
 }
 
 // |u| exactly as speed_kernel computes it (the same expression)
@@ -237,85 +286,90 @@ __device__ __forceinline__ float speed3(float u, float v, float w) {
 constexpr int LINES = 256;           // lines per block
 constexpr int MAXLINE = 39;          // "u v w\n" at 12 bytes per value
 
-template <int KIND>
-__device__ __forceinline__ int format_line(const float* a, const float* b, const float* c, int64_t i, char* buf) {
-    int len;
-    if (KIND == LBM_VTK_SCALAR) {
-        len = fmt_g6(a[i], buf);
-    } else if (KIND == LBM_VTK_SPEED) {
-        len = fmt_g6(speed3(a[i], b[i], c[i]), buf);
-    } else {
-        len = fmt_g6(a[i], buf);
-        buf[len++] = ' ';
-        len += fmt_g6(b[i], buf + len);
-        buf[len++] = ' ';
-        len += fmt_g6(c[i], buf + len);
-    }
-    buf[len++] = '\n';
-    return len;
+__device__ const double kPow10[23] = G6_POW10;
+
+// Place of a block in the text: state[k] of block k is LEN | its bytes once they
+// are known, SUM | the bytes of blocks 0 .. k once those are.  One warp looks back,
+// 32 blocks at a time, until it finds a SUM.  The wait is bounded: every block
+// looked at has started, so a wait that runs out means that the launch is broken;
+// the block then publishes BAD, as do all behind it, and writes nothing.
+constexpr uint64_t LEN = 1ull << 62, SUM = 2ull << 62, BAD = 3ull << 62, VAL = LEN - 1;
+constexpr int kPolls = 1 << 22;
+
+__device__ __forceinline__ uint64_t state_ld(const uint64_t* p) {
+    uint64_t v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void state_st(uint64_t* p, uint64_t v) {
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
-template <int KIND>
-__global__ void __launch_bounds__(LINES) vtk_count(const float* a, const float* b, const float* c, int64_t n,
-                                                   uint32_t* block_bytes) {
-    const int64_t i = (int64_t)blockIdx.x * LINES + threadIdx.x;
-    char buf[MAXLINE + 1];
-    uint32_t len = i < n ? (uint32_t)format_line<KIND>(a, b, c, i, buf) : 0u;
-    // block sum: warp shuffles, then one warp over the 8 warp sums
-    for (int o = 16; o; o >>= 1) len += __shfl_xor_sync(0xffffffffu, len, o);
-    __shared__ uint32_t ws[LINES / 32];
-    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = len;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t s = 0;
-        for (int k = 0; k < LINES / 32; ++k) s += ws[k];
-        block_bytes[blockIdx.x] = s;
+// called by one whole warp; returns the bytes before block `me`, or BAD
+__device__ uint64_t text_place(uint64_t* state, int64_t me, uint32_t total) {
+    const int lane = threadIdx.x & 31;
+    if (me == 0) {
+        if (lane == 0) state_st(state, SUM | total);
+        return 0;
     }
-}
-
-// exclusive scan of the block byte counts (one block of 1024 threads);
-// offsets[nb] receives the total
-__global__ void __launch_bounds__(1024) vtk_scan(const uint32_t* block_bytes, int64_t nb, uint64_t* offsets) {
-    __shared__ uint64_t ws[32];
-    __shared__ uint64_t carry;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    for (int64_t base = 0; base < nb; base += 1024) {
-        const int64_t j = base + threadIdx.x;
-        const uint64_t x = j < nb ? block_bytes[j] : 0u;
-        uint64_t s = x;   // inclusive warp scan
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint64_t y = __shfl_up_sync(0xffffffffu, s, o);
-            if ((threadIdx.x & 31) >= o) s += y;
+    if (lane == 0) state_st(state + me, LEN | total);
+    uint64_t before = 0;
+    for (int64_t end = me; end > 0;) {          // blocks end-32 .. end-1 are looked at, lane 0 the nearest
+        const int64_t j = end - 1 - lane;
+        uint64_t v = SUM;                        // (before the first block: a sum of nothing)
+        int polls = 0;
+        if (j >= 0)
+            while ((v = state_ld(state + j)) < LEN && ++polls < kPolls) __nanosleep(20);
+        const uint64_t kind = v & BAD;
+        if (__any_sync(0xffffffffu, kind == 0 || kind == BAD)) {
+            if (lane == 0) state_st(state + me, BAD);
+            return BAD;
         }
-        if ((threadIdx.x & 31) == 31) ws[threadIdx.x >> 5] = s;
-        __syncthreads();
-        if (threadIdx.x < 32) {
-            uint64_t t = ws[threadIdx.x];
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint64_t y = __shfl_up_sync(0xffffffffu, t, o);
-                if (threadIdx.x >= o) t += y;
-            }
-            ws[threadIdx.x] = t;
-        }
-        __syncthreads();
-        const uint64_t before = carry + (threadIdx.x >= 32 ? ws[(threadIdx.x >> 5) - 1] : 0u) + s - x;
-        if (j < nb) offsets[j] = before;
-        __syncthreads();
-        if (threadIdx.x == 1023) carry = before + x;
-        __syncthreads();
+        const uint32_t sums = __ballot_sync(0xffffffffu, kind == SUM);
+        const int stop = sums ? __ffs((int)sums) - 1 : 32;      // the nearest sum ends the walk
+        uint64_t add = lane <= stop ? (v & VAL) : 0;
+        for (int o = 16; o; o >>= 1) add += __shfl_xor_sync(0xffffffffu, add, o);
+        before += add;
+        if (sums) break;
+        end -= 32;
     }
-    if (threadIdx.x == 0) offsets[nb] = carry;
+    if (lane == 0) state_st(state + me, SUM | (before + total));
+    return before;
 }
 
+// Bound by integer and double arithmetic: about 40 instructions a value for the digits
+// and 60 for the characters, against 4-12 B read and 8-35 B written a line.
+// 256x128x128 (4.19 M lines): the two-kernel form, which formatted every value
+// twice through arrays in local memory, took 452 us for u v w.
 template <int KIND>
 __global__ void __launch_bounds__(LINES) vtk_emit(const float* a, const float* b, const float* c, int64_t n,
-                                                  const uint64_t* offsets, char* text) {
-    __shared__ char stage[LINES * MAXLINE + 16];
+                                                  uint32_t* ticket, uint64_t* state, int64_t nb, char* text) {
+    constexpr int NV = KIND == LBM_VTK_VECTOR ? 3 : 1;
+    __shared__ __align__(16) char stage[LINES * (KIND == LBM_VTK_VECTOR ? MAXLINE : 13) + 16];
     __shared__ uint32_t ws[LINES / 32];
-    const int64_t i = (int64_t)blockIdx.x * LINES + threadIdx.x;
-    char buf[MAXLINE + 1];
-    const uint32_t len = i < n ? (uint32_t)format_line<KIND>(a, b, c, i, buf) : 0u;
+    __shared__ uint32_t block;
+    __shared__ uint64_t place;
+    __shared__ double p10[23];
+    if (threadIdx.x == 0) block = atomicAdd(ticket, 1u);
+    if (threadIdx.x < 23) p10[threadIdx.x] = kPow10[threadIdx.x];
+    __syncthreads();
+    const int64_t me = block;
+    const int64_t i = me * LINES + threadIdx.x;
+    G6 g[NV];
+    uint32_t len = 0;
+    if (i < n) {
+        if (KIND == LBM_VTK_SCALAR) {
+            g[0] = g6_parse(a[i], p10);
+        } else if (KIND == LBM_VTK_SPEED) {
+            g[0] = g6_parse(speed3(a[i], b[i], c[i]), p10);
+        } else {
+            const float v[3] = {a[i], b[i], c[i]};
+#pragma unroll
+            for (int k = 0; k < NV; ++k) g[k] = g6_parse(v[k], p10);
+        }
+#pragma unroll
+        for (int k = 0; k < NV; ++k) len += (uint32_t)g6_len(g[k]) + 1u;      // a blank or the line's end behind each
+    }
     // exclusive scan of the line lengths inside the block
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t s = len;
@@ -325,25 +379,38 @@ __global__ void __launch_bounds__(LINES) vtk_emit(const float* a, const float* b
     }
     if (lane == 31) ws[warp] = s;
     __syncthreads();
-    uint32_t wbase = 0;
-    for (int k = 0; k < warp; ++k) wbase += ws[k];
-    const uint32_t off = wbase + s - len;
-    for (uint32_t k = 0; k < len; ++k) stage[off + k] = buf[k];
-    uint32_t total = 0;
-    for (int k = 0; k < LINES / 32; ++k) total += ws[k];
+    uint32_t wbase = 0, total = 0;
+    for (int k = 0; k < LINES / 32; ++k) {
+        if (k < warp) wbase += ws[k];
+        total += ws[k];
+    }
+    if (warp == 0) {
+        const uint64_t at = text_place(state, me, total);
+        if (lane == 0) {
+            place = at;
+            if (me == nb - 1) state[nb] = at == BAD ? ~0ull : at + total;
+        }
+    }
+    if (i < n) {
+        char* o = stage + wbase + s - len;
+#pragma unroll
+        for (int k = 0; k < NV; ++k) {
+            o += g6_put(g[k], o);
+            *o++ = k == NV - 1 ? '\n' : ' ';
+        }
+    }
     __syncthreads();
+    if (place == BAD) return;
     // block text -> global: bytes up to a 4-byte boundary, words, then the tail
-    const uint64_t dst = offsets[blockIdx.x];
+    const uint64_t dst = place;
     const uint32_t head = (uint32_t)((4u - (uint32_t)(dst & 3u)) & 3u);
     const uint32_t h = head < total ? head : total;
     if (threadIdx.x < h) text[dst + threadIdx.x] = stage[threadIdx.x];
     const uint32_t words = (total - h) >> 2;
     uint32_t* tw = reinterpret_cast<uint32_t*>(text + dst + h);
-    for (uint32_t k = threadIdx.x; k < words; k += LINES) {
-        const uint32_t p = h + 4u * k;
-        tw[k] = (uint32_t)(uint8_t)stage[p] | ((uint32_t)(uint8_t)stage[p + 1] << 8) |
-                ((uint32_t)(uint8_t)stage[p + 2] << 16) | ((uint32_t)(uint8_t)stage[p + 3] << 24);
-    }
+    const uint32_t* sw = reinterpret_cast<const uint32_t*>(stage);
+    for (uint32_t k = threadIdx.x; k < words; k += LINES)
+        tw[k] = h == 0 ? sw[k] : __funnelshift_r(sw[k], sw[k + 1], 8u * h);
     const uint32_t t0 = h + 4u * words;
     if (threadIdx.x < total - t0) text[dst + t0 + threadIdx.x] = stage[t0 + threadIdx.x];
 }
@@ -351,21 +418,18 @@ __global__ void __launch_bounds__(LINES) vtk_emit(const float* a, const float* b
 int64_t max_line(int kind) { return kind == LBM_VTK_VECTOR ? MAXLINE : 13; }
 
 // Queues the formatting of one field: text[0..total) on the device, total in
-// offsets[nb].  scratch: nb uint32 counts; offsets: nb + 1 uint64.
-cudaError_t launch_format(int kind, const float* a, const float* b, const float* c, int64_t n, uint32_t* counts,
-                          uint64_t* offsets, char* text, cudaStream_t st) {
+// state[nb] (all ones if a wait inside ran out).  ticket: one uint32; state: nb + 1
+// uint64, the blocks' lengths.
+cudaError_t launch_format(int kind, const float* a, const float* b, const float* c, int64_t n, uint32_t* ticket,
+                          uint64_t* state, char* text, cudaStream_t st) {
     const int64_t nb = (n + LINES - 1) / LINES;
-    if (nb == 0) return cudaMemsetAsync(offsets, 0, sizeof(uint64_t), st);
+    cudaError_t e = cudaMemsetAsync(ticket, 0, sizeof(uint32_t), st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(state, 0, sizeof(uint64_t) * (size_t)(nb + 1), st);
+    if (e != cudaSuccess || nb == 0) return e;
     switch (kind) {
-        case LBM_VTK_SCALAR: vtk_count<LBM_VTK_SCALAR><<<(unsigned)nb, LINES, 0, st>>>(a, b, c, n, counts); break;
-        case LBM_VTK_SPEED: vtk_count<LBM_VTK_SPEED><<<(unsigned)nb, LINES, 0, st>>>(a, b, c, n, counts); break;
-        default: vtk_count<LBM_VTK_VECTOR><<<(unsigned)nb, LINES, 0, st>>>(a, b, c, n, counts); break;
-    }
-    vtk_scan<<<1, 1024, 0, st>>>(counts, nb, offsets);
-    switch (kind) {
-        case LBM_VTK_SCALAR: vtk_emit<LBM_VTK_SCALAR><<<(unsigned)nb, LINES, 0, st>>>(a, b, c, n, offsets, text); break;
-        case LBM_VTK_SPEED: vtk_emit<LBM_VTK_SPEED><<<(unsigned)nb, LINES, 0, st>>>(a, b, c, n, offsets, text); break;
-        default: vtk_emit<LBM_VTK_VECTOR><<<(unsigned)nb, LINES, 0, st>>>(a, b, c, n, offsets, text); break;
+        case LBM_VTK_SCALAR: vtk_emit<LBM_VTK_SCALAR><<<(unsigned)nb, LINES, 0, st>>>(a, b, c, n, ticket, state, nb, text); break;
+        case LBM_VTK_SPEED: vtk_emit<LBM_VTK_SPEED><<<(unsigned)nb, LINES, 0, st>>>(a, b, c, n, ticket, state, nb, text); break;
+        default: vtk_emit<LBM_VTK_VECTOR><<<(unsigned)nb, LINES, 0, st>>>(a, b, c, n, ticket, state, nb, text); break;
     }
     return cudaGetLastError();
 }
@@ -425,8 +489,8 @@ using namespace lbm::vtk;
 struct lbm_vtk_writer {
     struct Slot {
         char* d_text = nullptr;
-        uint32_t* d_counts = nullptr;
-        uint64_t* d_offsets = nullptr;
+        uint32_t* d_ticket = nullptr;
+        uint64_t* d_state = nullptr;
         cudaEvent_t formatted = nullptr;
         bool busy = false;
     };
@@ -460,12 +524,13 @@ struct lbm_vtk_writer {
     void write_job(const Job& j) {
         Slot& s = slots[j.slot];
         if (cudaEventSynchronize(s.formatted) != cudaSuccess ||
-            cudaMemcpyAsync(h_total, s.d_offsets + nb, sizeof(uint64_t), cudaMemcpyDeviceToHost, copy) != cudaSuccess ||
+            cudaMemcpyAsync(h_total, s.d_state + nb, sizeof(uint64_t), cudaMemcpyDeviceToHost, copy) != cudaSuccess ||
             cudaStreamSynchronize(copy) != cudaSuccess) {
             fail(LBM_ERR_CUDA, "vtk writer: formatting or copy failed");
             return;
         }
         const uint64_t total = *h_total;
+        if (total > (uint64_t)cap) { fail(LBM_ERR_TIMEOUT, "vtk writer: a wait in the formatting kernel ran out"); return; }
         FILE* f = std::fopen(j.path.c_str(), "wb");
         if (!f) { fail(LBM_ERR_IO, "failed to open VTK file: " + j.path); return; }
         const std::string h = header(j.kind, nx, ny, nz);
@@ -535,8 +600,8 @@ int lbm_vtk_writer_create(int32_t nx, int32_t ny, int32_t nz, int32_t depth, lbm
     w->slots.resize((size_t)(depth < 1 ? 1 : depth));
     for (auto& s : w->slots) {
         ok = ok && cudaMalloc((void**)&s.d_text, (size_t)w->cap + 16) == cudaSuccess &&
-             cudaMalloc((void**)&s.d_counts, sizeof(uint32_t) * (size_t)(w->nb + 1)) == cudaSuccess &&
-             cudaMalloc((void**)&s.d_offsets, sizeof(uint64_t) * (size_t)(w->nb + 1)) == cudaSuccess &&
+             cudaMalloc((void**)&s.d_ticket, sizeof(uint32_t)) == cudaSuccess &&
+             cudaMalloc((void**)&s.d_state, sizeof(uint64_t) * (size_t)(w->nb + 1)) == cudaSuccess &&
              cudaEventCreateWithFlags(&s.formatted, cudaEventDisableTiming) == cudaSuccess;
     }
     if (!ok) {
@@ -568,7 +633,7 @@ int lbm_vtk_writer_submit(lbm_vtk_writer* w, int32_t kind, const float* d_a, con
     }
     auto& s = w->slots[slot];
     const cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (launch_format(kind, d_a, d_b, d_c, w->n, s.d_counts, s.d_offsets, s.d_text, st) != cudaSuccess ||
+    if (launch_format(kind, d_a, d_b, d_c, w->n, s.d_ticket, s.d_state, s.d_text, st) != cudaSuccess ||
         cudaEventRecord(s.formatted, st) != cudaSuccess) {
         std::lock_guard<std::mutex> g(w->mu);
         s.busy = false;
@@ -614,7 +679,7 @@ int lbm_vtk_writer_destroy(lbm_vtk_writer* w) {
         w->th.join();
     }
     for (auto& s : w->slots) {
-        cudaFree(s.d_text); cudaFree(s.d_counts); cudaFree(s.d_offsets);
+        cudaFree(s.d_text); cudaFree(s.d_ticket); cudaFree(s.d_state);
         if (s.formatted) cudaEventDestroy(s.formatted);
     }
     if (w->h_text) cudaFreeHost(w->h_text);
@@ -637,22 +702,19 @@ int lbm_vtk_format(int32_t kind, const float* d_a, const float* d_b, const float
     if (cap < lbm_vtk_text_bound(kind, n)) { lbm::set_error("lbm_vtk_format: text buffer too small"); return LBM_ERR_INVALID; }
     const int64_t nb = (n + LINES - 1) / LINES;
     const cudaStream_t st = static_cast<cudaStream_t>(stream);
-    // scratch from the stream-ordered pool: no device-wide synchronisation
-    uint32_t* counts = nullptr;
-    uint64_t* offsets = nullptr;
-    if (cudaMallocAsync((void**)&counts, sizeof(uint32_t) * (size_t)(nb + 1), st) != cudaSuccess ||
-        cudaMallocAsync((void**)&offsets, sizeof(uint64_t) * (size_t)(nb + 1), st) != cudaSuccess) {
-        if (counts) cudaFreeAsync(counts, st);
+    uint64_t* scratch = nullptr;      // the blocks' lengths, the total, the ticket
+    if (lbm::scratch_alloc((void**)&scratch, sizeof(uint64_t) * (size_t)(nb + 2), st) != cudaSuccess) {
         lbm::set_error("lbm_vtk_format: allocation failed");
         return LBM_ERR_ALLOC;
     }
     uint64_t total = 0;
-    const bool ok = launch_format(kind, d_a, d_b, d_c, n, counts, offsets, d_text, st) == cudaSuccess &&
-                    cudaMemcpyAsync(&total, offsets + nb, sizeof(uint64_t), cudaMemcpyDeviceToHost, st) == cudaSuccess;
-    cudaFreeAsync(counts, st);
-    cudaFreeAsync(offsets, st);
+    const bool ok = launch_format(kind, d_a, d_b, d_c, n, reinterpret_cast<uint32_t*>(scratch + nb + 1), scratch, d_text,
+                                  st) == cudaSuccess &&
+                    cudaMemcpyAsync(&total, scratch + nb, sizeof(uint64_t), cudaMemcpyDeviceToHost, st) == cudaSuccess;
+    cudaFreeAsync(scratch, st);
     if (cudaStreamSynchronize(st) != cudaSuccess) { lbm::set_error("lbm_vtk_format: kernel failed"); return LBM_ERR_CUDA; }
     if (!ok) { lbm::set_error("lbm_vtk_format: kernel failed"); return LBM_ERR_CUDA; }
+    if (total > (uint64_t)cap) { lbm::set_error("lbm_vtk_format: a wait in the kernel ran out"); return LBM_ERR_TIMEOUT; }
     *len = (int64_t)total;
     return LBM_OK;
 }

@@ -68,6 +68,21 @@ def test_device_text_equals_host_formatter(gpu, n):
     assert format_device(VTK_SPEED, du, dv, dw) == lines(VTK_SCALAR, speed_of(u, v, w)).encode()
 
 
+@pytest.mark.parametrize("n", [8191, 256 * 33 + 1, 256 * 70])
+def test_text_of_every_length_is_placed(gpu, n):
+    """Line lengths from 2 to 39 bytes in blocks of 256 lines: the place of every block, 32 blocks and more looked
+    back over, all four alignments of a block's start, and values that take the exact path."""
+    rng = np.random.default_rng(n)
+    f = [(rng.standard_normal(n) * 10.0 ** rng.integers(-9, 9, n)).astype(np.float32) for _ in range(3)]
+    for a in f:
+        a[rng.integers(0, n, n // 3)] = 0.0
+        a[rng.integers(0, n, n // 5)] = rng.choice(np.array([1.0, 0.5, 999999.5, 100000.5, -1e-5, 1e22, 3e-39], np.float32),
+                                                   n // 5)
+    t = [torch.from_numpy(a).cuda() for a in f]
+    assert format_device(VTK_SCALAR, t[0]) == lines(VTK_SCALAR, f[0]).encode()
+    assert format_device(VTK_VECTOR, *t) == lines(VTK_VECTOR, *f).encode()
+
+
 def test_empty_field(gpu):
     z = torch.empty(0, device="cuda")
     assert format_device(VTK_SCALAR, z) == b""
