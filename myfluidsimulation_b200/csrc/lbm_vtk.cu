@@ -148,17 +148,27 @@ HD uint32_t scaled_floor(uint32_t m, int e, int s, int& half) {
     {1e0, 1e1, 1e2, 1e3, 1e4, 1e5, 1e6, 1e7, 1e8, 1e9, 1e10, 1e11, 1e12, 1e13, 1e14, 1e15, 1e16, 1e17, 1e18, 1e19, \
      1e20, 1e21, 1e22}
 
-// A value as printf("%g") shows it: six digits n (100000 .. 999999), decimal
-// exponent x, sign, and kind 0 (a number), 1 (zero), 2 (inf), 3 (nan).
+// A value as printf("%g") shows it: its six digits (a byte each, the first in the
+// lowest byte), decimal exponent x, sign, and kind 0 (a number), 1 (zero), 2 (inf),
+// 3 (nan); last: index of the last digit kept (trailing zeros are dropped).
 struct G6 {
-    uint32_t n;
+    uint64_t d;
     int8_t x;
-    uint8_t neg, kind;
-    uint8_t last;      // index of the last digit kept (trailing zeros are dropped)
+    uint8_t neg, kind, last;
 };
 
+// six digits of n < 10^6, a byte each, the first in the lowest byte
+HD uint64_t g6_digits(uint32_t n) {
+    const uint32_t hi = n / 1000u, lo = n - hi * 1000u;
+    auto three = [](uint32_t v) {      // v < 1000
+        const uint32_t a = v / 100u, r = v - a * 100u, b = r / 10u;
+        return a | (b << 8) | ((r - b * 10u) << 16);
+    };
+    return (uint64_t)three(hi) | ((uint64_t)three(lo) << 24);
+}
+
 // the digits by exact integer comparison: values next to a rounding or digit boundary
-HD void g6_exact(uint32_t m, int e, int& X, uint32_t& n, int& half) {
+__host__ __device__ __noinline__ void g6_exact(uint32_t m, int e, int& X, uint32_t& n, int& half) {
     for (int it = 0; it < 4; ++it) {
         n = scaled_floor(m, e, 5 - X, half);
         if (n >= 1000000u) { ++X; continue; }
@@ -194,6 +204,8 @@ HD G6 g6_parse(float v, const double* p10) {
     // or far enough from both), else the exact path below decides
     const double x = (double)(bits >> 31 ? -v : v);
     bool done = false;
+    // the estimate is X or X - 1: settle it by comparison where both powers are at hand
+    if (X >= -16 && X <= 4 && x * p10[5 - X] >= 1000000.0) ++X;
     for (int it = 0; it < 3; ++it) {
         const int k = 5 - X;
         if (k < -22 || k > 22) break;
@@ -210,17 +222,22 @@ HD G6 g6_parse(float v, const double* p10) {
         done = true;
         break;
     }
-    if (!done) g6_exact(m, e, X, n, half);
+    if (!done) {
+        int xe = X, he = 0;
+        uint32_t ne = 0;
+        g6_exact(m, e, xe, ne, he);      // (its results by address: X, n and half stay in registers)
+        X = xe; n = ne; half = he;
+    }
     if (half > 0 || (half == 0 && (n & 1u))) {
         if (++n == 1000000u) { n = 100000u; ++X; }
     }
-    g.n = n;
+    g.d = g6_digits(n);
     g.x = (int8_t)X;
-    // trailing zeros
-    uint32_t r = n;
-    int last = 5;
-    while (last > 0 && r % 10u == 0u) { r /= 10u; --last; }
-    g.last = (uint8_t)last;
+#ifdef __CUDA_ARCH__
+    g.last = (uint8_t)((63 - __clzll((long long)g.d)) >> 3);
+#else
+    g.last = (uint8_t)((63 - __builtin_clzll(g.d)) >> 3);
+#endif
     return g;
 }
 
@@ -234,47 +251,63 @@ HD int g6_len(const G6& g) {
     return neg + 2 + (-X - 1) + last + 1;
 }
 
-// the characters of g into out (at most 12); returns their number
-HD int g6_put(const G6& g, char* out) {
-    char* o = out;
-    if (g.neg) *o++ = '-';
+// up to 16 characters, the first in the lowest byte of lo
+struct Text {
+    uint64_t lo, hi;
+    int len;
+};
+// the k characters of v behind those of t (k <= 8; v holds nothing above them)
+HD void text_add(Text& t, uint64_t v, int k) {
+    if (t.len < 8) {
+        t.lo |= v << (8 * t.len);
+        if (t.len > 0) t.hi |= v >> (64 - 8 * t.len);
+    } else {
+        t.hi |= v << (8 * (t.len - 8));
+    }
+    t.len += k;
+}
+
+// the characters of g, at most 12: [-] digits with a point behind digit x (0 in
+// exponent form, or "0." and zeros in front of all), [e+dd]
+HD Text g6_text(const G6& g) {
+    Text t{0, 0, 0};
+    if (g.neg) text_add(t, '-', 1);
     if (g.kind) {
-        if (g.kind == 1) { *o++ = '0'; return (int)(o - out); }
-        const bool nan = g.kind == 3;
-        *o++ = nan ? 'n' : 'i'; *o++ = nan ? 'a' : 'n'; *o++ = nan ? 'n' : 'f';
-        return (int)(o - out);
+        if (g.kind == 1) text_add(t, '0', 1);
+        else text_add(t, g.kind == 3 ? 0x6e616eull : 0x666e69ull, 3);      // "nan", "inf"
+        return t;
     }
     const int X = g.x, last = g.last;
-    // where the point goes: behind digit `point` (-1: in front of all, after "0." and zeros)
+    const uint64_t dg = g.d + 0x303030303030ull;
     const bool ex = X < -4 || X >= 6;
     const int point = ex ? 0 : X;
     if (point < 0) {
-        *o++ = '0';
-        *o++ = '.';
-        for (int i = 0; i < -X - 1; ++i) *o++ = '0';
+        text_add(t, 0x3030302e30ull & ((1ull << (8 * (1 - point))) - 1), 1 - point);      // "0." and -X-1 zeros
+        text_add(t, dg & ((1ull << (8 * (last + 1))) - 1), last + 1);
+    } else {
+        const int in = point + 1;                                          // digits before the point
+        const uint64_t low = dg & ((1ull << (8 * in)) - 1);
+        if (last > point) {
+            const uint64_t frac = (dg >> (8 * in)) & ((1ull << (8 * (last - point))) - 1);
+            text_add(t, low | ((uint64_t)'.' << (8 * in)) | (frac << (8 * (in + 1))), last + 2);
+        } else {
+            text_add(t, low, in);
+        }
+        if (ex) {
+            const int a = X < 0 ? -X : X, tens = a / 10;
+            text_add(t, 'e' | ((X < 0 ? '-' : '+') << 8) | ((uint64_t)('0' + tens) << 16) |
+                            ((uint64_t)('0' + a - 10 * tens) << 24), 4);
+        }
     }
-    uint32_t r = g.n, p = 100000u;
-    for (int i = 0; i < 6; ++i) {
-        const uint32_t d = r / p;
-        r -= d * p;
-        p /= 10u;
-        if (i <= last || i <= point) *o++ = (char)('0' + d);
-        if (i == point && last > point) *o++ = '.';
-    }
-    if (ex) {
-        *o++ = 'e';
-        *o++ = X < 0 ? '-' : '+';
-        const int a = X < 0 ? -X : X;
-        *o++ = (char)('0' + a / 10);
-        *o++ = (char)('0' + a % 10);
-    }
-    return (int)(o - out);
+    return t;
 }
 
 // Bytes of printf("%g", (double)v) into out (at most 12); returns the length.
 inline int fmt_g6(float v, char* out) {
     static const double p10[23] = G6_POW10;
-    return g6_put(g6_parse(v, p10), out);
+    const Text t = g6_text(g6_parse(v, p10));
+    for (int i = 0; i < t.len; ++i) out[i] = (char)((i < 8 ? t.lo >> (8 * i) : t.hi >> (8 * (i - 8))) & 0xff);
+    return t.len;
 }
 
 // |u| exactly as speed_kernel computes it (the same expression)
@@ -305,14 +338,10 @@ __device__ __forceinline__ void state_st(uint64_t* p, uint64_t v) {
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
-// called by one whole warp; returns the bytes before block `me`, or BAD
+// called by one whole warp once the block has published its length (block 0: its sum); returns the bytes before block `me`, or BAD
 __device__ uint64_t text_place(uint64_t* state, int64_t me, uint32_t total) {
     const int lane = threadIdx.x & 31;
-    if (me == 0) {
-        if (lane == 0) state_st(state, SUM | total);
-        return 0;
-    }
-    if (lane == 0) state_st(state + me, LEN | total);
+    if (me == 0) return 0;
     uint64_t before = 0;
     for (int64_t end = me; end > 0;) {          // blocks end-32 .. end-1 are looked at, lane 0 the nearest
         const int64_t j = end - 1 - lane;
@@ -337,12 +366,13 @@ __device__ uint64_t text_place(uint64_t* state, int64_t me, uint32_t total) {
     return before;
 }
 
-// Bound by integer and double arithmetic: about 40 instructions a value for the digits
-// and 60 for the characters, against 4-12 B read and 8-35 B written a line.
-// 256x128x128 (4.19 M lines): the two-kernel form, which formatted every value
-// twice through arrays in local memory, took 452 us for u v w.
+// Bound by issue slots: about 440 instructions a value (a third of them integer
+// multiplies, shifts and tests of the digits and the text), against 4-12 B read and
+// 8-35 B written a line.  u v w of 256x128x128 cells (4.19 M lines): 242 us, from 452
+// in the two-kernel form that formatted every value twice through arrays in local
+// memory; looking back before the text is made, instead of behind it, 315 us.
 template <int KIND>
-__global__ void __launch_bounds__(LINES) vtk_emit(const float* a, const float* b, const float* c, int64_t n,
+__global__ void __launch_bounds__(LINES, 4) vtk_emit(const float* a, const float* b, const float* c, int64_t n,
                                                   uint32_t* ticket, uint64_t* state, int64_t nb, char* text) {
     constexpr int NV = KIND == LBM_VTK_VECTOR ? 3 : 1;
     __shared__ __align__(16) char stage[LINES * (KIND == LBM_VTK_VECTOR ? MAXLINE : 13) + 16];
@@ -384,19 +414,47 @@ __global__ void __launch_bounds__(LINES) vtk_emit(const float* a, const float* b
         if (k < warp) wbase += ws[k];
         total += ws[k];
     }
+    if (threadIdx.x == 0) state_st(state + me, (me == 0 ? SUM : LEN) | total);
+    // the line's characters in words: whole words are stored as such, and a word that the
+    // line shares with its neighbours byte by byte
+    if (i < n) {
+        uint32_t at = wbase + s - len;
+        uint64_t acc = 0;
+        uint32_t fill = at & 3u;              // bytes of the current word before and in acc
+        uint32_t skip = fill;                 // of them, the neighbour's
+        uint32_t* w = reinterpret_cast<uint32_t*>(stage) + (at >> 2);
+#pragma unroll
+        for (int k = 0; k < NV; ++k) {
+            Text t = g6_text(g[k]);
+            text_add(t, k == NV - 1 ? '\n' : ' ', 1);
+            const uint32_t part[4] = {(uint32_t)t.lo, (uint32_t)(t.lo >> 32), (uint32_t)t.hi, (uint32_t)(t.hi >> 32)};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int m = min(max(t.len - 4 * j, 0), 4);
+                acc |= (uint64_t)part[j] << (8u * fill);
+                fill += (uint32_t)m;
+                if (fill >= 4u) {
+                    if (skip) {
+                        char* o = reinterpret_cast<char*>(w);
+                        for (uint32_t q = skip; q < 4u; ++q) o[q] = (char)(acc >> (8u * q));
+                        skip = 0;
+                    } else {
+                        *w = (uint32_t)acc;
+                    }
+                    ++w;
+                    acc >>= 32;
+                    fill -= 4u;
+                }
+            }
+        }
+        char* o = reinterpret_cast<char*>(w);
+        for (uint32_t q = skip; q < fill; ++q) o[q] = (char)(acc >> (8u * q));
+    }
     if (warp == 0) {
         const uint64_t at = text_place(state, me, total);
         if (lane == 0) {
             place = at;
             if (me == nb - 1) state[nb] = at == BAD ? ~0ull : at + total;
-        }
-    }
-    if (i < n) {
-        char* o = stage + wbase + s - len;
-#pragma unroll
-        for (int k = 0; k < NV; ++k) {
-            o += g6_put(g[k], o);
-            *o++ = k == NV - 1 ? '\n' : ' ';
         }
     }
     __syncthreads();
