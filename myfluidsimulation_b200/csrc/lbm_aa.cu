@@ -299,6 +299,7 @@ __device__ __forceinline__ void even_unit(const AAParams& p, IDX v, double (&acc
 template <class ST, bool MASK, int VEC, int MODE, class IDX>
 __global__ void __launch_bounds__(256, 2) aa_even(AAParams p) {
     constexpr bool STATS = MODE == 2;
+    step_begin();
     const IDX v0 = (IDX)(p.first / VEC), v1 = (IDX)((p.first + p.cells) / VEC);
     double acc[NSTAT];
 #pragma unroll
@@ -476,6 +477,7 @@ struct NbrZ {
 template <class ST, int MODE, class IDX>
 __global__ void __launch_bounds__(256, ST::kId == 3 ? 2 : 3) aa_odd(AAParams p) {
     constexpr bool STATS = MODE == 2;
+    step_begin();
     const int segs = (p.nx + p.bx - 1) / p.bx;
     const int yblocks = (p.ny + p.by - 1) / p.by;
     const IDX plane = (IDX)p.nx * (IDX)p.ny;
@@ -515,6 +517,7 @@ __global__ void __launch_bounds__(256, ST::kId == 3 ? 2 : 3) aa_odd(AAParams p) 
 template <class ST, int MODE, class IDX>
 __global__ void __launch_bounds__(256, ST::kId == 3 ? 2 : 4) aa_odd_rows(AAParams p) {
     constexpr bool STATS = MODE == 2;
+    step_begin();
     const int ty = (int)threadIdx.x / p.bx;
     const int x = (int)blockIdx.y * p.bx + (int)threadIdx.x - ty * p.bx;
     const int rows = (int)(p.cells / p.nx);
@@ -619,14 +622,14 @@ void launch_mode(const AAParams& p, int parity, LaunchCfg cfg, cudaStream_t s) {
     if (parity == 0) {
         const int64_t span = p.first | p.cells;      // both must be multiples of the vector width
         if (V == 4 && span % 4 != 0 && span % 2 == 0) {
-            if (mask) aa_even<ST, true, 2, MODE, IDX><<<cfg.blocks, cfg.threads, 0, s>>>(p);
-            else aa_even<ST, false, 2, MODE, IDX><<<cfg.blocks, cfg.threads, 0, s>>>(p);
+            if (mask) launch_after(aa_even<ST, true, 2, MODE, IDX>, cfg.blocks, cfg.threads, 0, s, p);
+            else launch_after(aa_even<ST, false, 2, MODE, IDX>, cfg.blocks, cfg.threads, 0, s, p);
         } else if (span % V == 0) {
-            if (mask) aa_even<ST, true, V, MODE, IDX><<<cfg.blocks, cfg.threads, 0, s>>>(p);
-            else aa_even<ST, false, V, MODE, IDX><<<cfg.blocks, cfg.threads, 0, s>>>(p);
+            if (mask) launch_after(aa_even<ST, true, V, MODE, IDX>, cfg.blocks, cfg.threads, 0, s, p);
+            else launch_after(aa_even<ST, false, V, MODE, IDX>, cfg.blocks, cfg.threads, 0, s, p);
         } else {
-            if (mask) aa_even<ST, true, 1, MODE, IDX><<<cfg.blocks, cfg.threads, 0, s>>>(p);
-            else aa_even<ST, false, 1, MODE, IDX><<<cfg.blocks, cfg.threads, 0, s>>>(p);
+            if (mask) launch_after(aa_even<ST, true, 1, MODE, IDX>, cfg.blocks, cfg.threads, 0, s, p);
+            else launch_after(aa_even<ST, false, 1, MODE, IDX>, cfg.blocks, cfg.threads, 0, s, p);
         }
     } else {
         AAParams q = p;
@@ -635,14 +638,14 @@ void launch_mode(const AAParams& p, int parity, LaunchCfg cfg, cudaStream_t s) {
         if (mask) {
             const int segs = (p.nx + q.bx - 1) / q.bx;
             const dim3 grid((unsigned)std::max(1, cfg.blocks / segs), (unsigned)segs);
-            aa_odd_rows<ST, MODE, IDX><<<grid, threads, 0, s>>>(q);
+            launch_after(aa_odd_rows<ST, MODE, IDX>, grid, threads, 0, s, q);
             return;
         }
         const int64_t planes = p.cells / ((int64_t)p.nx * p.ny);
         q.zrun = aa_odd_zrun(p.nx, p.ny, planes, ST::kId, cfg.threads);
         const int64_t blocks = aa_odd_blocks(p.nx, p.ny, planes, ST::kId, cfg.threads);
         if (blocks <= 0) return;
-        aa_odd<ST, MODE, IDX><<<(unsigned)blocks, threads, 0, s>>>(q);
+        launch_after(aa_odd<ST, MODE, IDX>, (unsigned)blocks, threads, 0, s, q);
     }
 }
 

@@ -145,6 +145,7 @@ __global__ void adj_init(AdjP<R> p, const double* __restrict__ u0, R* __restrict
 template <class R, class IDX>
 __global__ void __launch_bounds__(256) adj_fwd(AdjP<R> p, const R* __restrict__ f, R* __restrict__ fn,
                                                const double* __restrict__ uin, double* __restrict__ drag_part) {
+    step_begin();
     double drag = 0.0;
     const IDX N = (IDX)p.N;
     const int64_t id64 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -226,6 +227,7 @@ template <class R, class IDX>
 __global__ void __launch_bounds__(256) adj_bwd(AdjP<R> p, const R* __restrict__ f, const R* __restrict__ lam1,
                                                R* __restrict__ lam0, const double* __restrict__ uin,
                                                double* __restrict__ g_uin, R wdrag) {
+    step_begin();
     const IDX N = (IDX)p.N;
     const int64_t id64 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (id64 >= p.N) return;
@@ -357,15 +359,15 @@ struct AdjBuffers {
 template <class R>
 void run_fwd(const AdjP<R>& p, const R* f, R* fn, const double* uin, double* drag, cudaStream_t s) {
     // 32-bit element offsets while every slot index 19*N fits in them
-    if ((uint64_t)p.N * 19u < (1ull << 32)) adj_fwd<R, uint32_t><<<blocks_for(p.N), 256, 0, s>>>(p, f, fn, uin, drag);
-    else adj_fwd<R, int64_t><<<blocks_for(p.N), 256, 0, s>>>(p, f, fn, uin, drag);
+    if ((uint64_t)p.N * 19u < (1ull << 32)) launch_after(adj_fwd<R, uint32_t>, blocks_for(p.N), 256, 0, s, p, f, fn, uin, drag);
+    else launch_after(adj_fwd<R, int64_t>, blocks_for(p.N), 256, 0, s, p, f, fn, uin, drag);
 }
 template <class R>
 void run_bwd(const AdjP<R>& p, const R* f, const R* lam1, R* lam0, const double* uin, double* guin, R wd,
              cudaStream_t s) {
     if ((uint64_t)p.N * 19u < (1ull << 32))
-        adj_bwd<R, uint32_t><<<blocks_for(p.N), 256, 0, s>>>(p, f, lam1, lam0, uin, guin, wd);
-    else adj_bwd<R, int64_t><<<blocks_for(p.N), 256, 0, s>>>(p, f, lam1, lam0, uin, guin, wd);
+        launch_after(adj_bwd<R, uint32_t>, blocks_for(p.N), 256, 0, s, p, f, lam1, lam0, uin, guin, wd);
+    else launch_after(adj_bwd<R, int64_t>, blocks_for(p.N), 256, 0, s, p, f, lam1, lam0, uin, guin, wd);
 }
 
 template <class R>

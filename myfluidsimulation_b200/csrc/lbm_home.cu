@@ -346,6 +346,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 8 ? 2 : 4) home_step(HomePara
     using E = typename HomeTypes<T>::E;
     using V = typename HomeTypes<T>::V;
     extern __shared__ __align__(16) unsigned char smraw[];
+    step_begin();
     E* sm = reinterpret_cast<E*>(smraw);
     const T* __restrict__ m = static_cast<const T*>(p.m);
     T* __restrict__ mn = static_cast<T*>(p.mn);
@@ -649,11 +650,11 @@ void launch_step(const HomeParams& p, cudaStream_t s) {
     // 32-bit element offsets while every index 10*N fits in them
     const bool slab = p.zb != 0 || p.ze != p.nz || p.salt_base != 0;
     if ((uint64_t)p.N * 10u < (1ull << 32)) {
-        if (slab) home_step<T, STATS, uint32_t, true><<<grid, NT, smem, s>>>(p);
-        else home_step<T, STATS, uint32_t, false><<<grid, NT, smem, s>>>(p);
+        if (slab) launch_after(home_step<T, STATS, uint32_t, true>, grid, NT, smem, s, p);
+        else launch_after(home_step<T, STATS, uint32_t, false>, grid, NT, smem, s, p);
     } else {
-        if (slab) home_step<T, STATS, int64_t, true><<<grid, NT, smem, s>>>(p);
-        else home_step<T, STATS, int64_t, false><<<grid, NT, smem, s>>>(p);
+        if (slab) launch_after(home_step<T, STATS, int64_t, true>, grid, NT, smem, s, p);
+        else launch_after(home_step<T, STATS, int64_t, false>, grid, NT, smem, s, p);
     }
 }
 

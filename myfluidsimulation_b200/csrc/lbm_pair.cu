@@ -75,6 +75,7 @@ template <bool VEC>
 __global__ void __launch_bounds__(NT, NB) aa_pair(AAParams p, const float* __restrict__ fa, float* __restrict__ fb,
                                                   int zchunk) {
     extern __shared__ __align__(16) float sm[];
+    step_begin();
     const int nx = p.nx, ny = p.ny, nz = p.nz;
     const int tiles_x = (nx + TX - 1) / TX, tiles_y = (ny + TY - 1) / TY;
     int b = blockIdx.x;
@@ -249,9 +250,8 @@ int pair_zchunk(int nx, int ny, int nz, int storage) {
 cudaError_t launch_aa_pair(const AAParams& p, const float* fa, float* fb, int zchunk, cudaStream_t s) {
     const int grid = ((p.nx + TX - 1) / TX) * ((p.ny + TY - 1) / TY) * ((p.nz + zchunk - 1) / zchunk);
     const size_t smem = sizeof(float) * SMEM_FLOATS;
-    if (p.nx % 2 == 0) aa_pair<true><<<grid, NT, smem, s>>>(p, fa, fb, zchunk);
-    else aa_pair<false><<<grid, NT, smem, s>>>(p, fa, fb, zchunk);
-    return cudaGetLastError();
+    return p.nx % 2 == 0 ? launch_after(aa_pair<true>, grid, NT, smem, s, p, fa, fb, zchunk)
+                         : launch_after(aa_pair<false>, grid, NT, smem, s, p, fa, fb, zchunk);
 }
 
 cudaError_t pair_prepare() {

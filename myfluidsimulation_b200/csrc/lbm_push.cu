@@ -43,6 +43,7 @@ __host__ __device__ constexpr uint32_t far_bit(int q) {
 template <int MODE, class IDX>
 __global__ void __launch_bounds__(256, 4) ref_push(AAParams p, const float* __restrict__ fa, float* __restrict__ fb) {
     constexpr bool MACRO = MODE >= 1, STATS = MODE == 2;
+    step_begin();
     const IDX N = (IDX)p.N;
     const int nx = p.nx, ny = p.ny, nz = p.nz;
     const uint8_t* __restrict__ fl = p.flags;
@@ -143,9 +144,9 @@ void push_idx(const AAParams& p, const float* fa, float* fb, LaunchCfg cfg, cuda
     // one block per 256 cells; with statistics the cfg.blocks whose partial sums the caller has room for
     const int64_t all = (p.N + cfg.threads - 1) / cfg.threads;
     const unsigned blocks = (unsigned)(all < ((int64_t)1 << 30) ? all : ((int64_t)1 << 30));
-    if (p.stats) ref_push<2, IDX><<<cfg.blocks, cfg.threads, 0, s>>>(p, fa, fb);
-    else if (p.macro) ref_push<1, IDX><<<blocks, cfg.threads, 0, s>>>(p, fa, fb);
-    else ref_push<0, IDX><<<blocks, cfg.threads, 0, s>>>(p, fa, fb);
+    if (p.stats) launch_after(ref_push<2, IDX>, cfg.blocks, cfg.threads, 0, s, p, fa, fb);
+    else if (p.macro) launch_after(ref_push<1, IDX>, blocks, cfg.threads, 0, s, p, fa, fb);
+    else launch_after(ref_push<0, IDX>, blocks, cfg.threads, 0, s, p, fa, fb);
 }
 
 }  // namespace
