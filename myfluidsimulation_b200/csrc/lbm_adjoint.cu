@@ -35,6 +35,7 @@
 #include "lbm_capi.h"
 #include "lbm_common.cuh"
 #include "lbm_internal.h"
+#include "lbm_vec.cuh"
 
 namespace lbm {
 void set_error(const std::string& msg);
@@ -104,29 +105,6 @@ struct AdjCell {
 };
 
 template <class R>
-struct AdjMom {
-    R rho, ux, uy, uz, uu;
-};
-template <class R>
-__device__ __forceinline__ AdjMom<R> adj_moments(const R (&fq)[19], const AdjP<R>& p) {
-    AdjMom<R> m;
-    R jx = 0, jy = 0, jz = 0;
-    m.rho = 0;
-    for_q<0, 19>([&](auto qi) {
-        constexpr int q = decltype(qi)::value;
-        m.rho += fq[q];
-        jx = plus_c<cx(q)>(jx, fq[q]);
-        jy = plus_c<cy(q)>(jy, fq[q]);
-        jz = plus_c<cz(q)>(jz, fq[q]);
-    });
-    m.ux = jx / m.rho + p.fx;
-    m.uy = jy / m.rho + p.fy;
-    m.uz = jz / m.rho + p.fz;
-    m.uu = m.ux * m.ux + m.uy * m.uy + m.uz * m.uz;
-    return m;
-}
-
-template <class R>
 __global__ void adj_init(AdjP<R> p, const double* __restrict__ u0, R* __restrict__ f) {
     for (int64_t id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; id < p.N; id += (int64_t)gridDim.x * blockDim.x) {
         const R ux = (R)u0[id], uy = (R)u0[p.N + id], uz = (R)u0[2 * p.N + id];
@@ -165,13 +143,8 @@ __global__ void __launch_bounds__(256) adj_fwd(AdjP<R> p, const R* __restrict__ 
         } else {
             AdjCell<IDX> c;
             c.init((uint32_t)id64, p.nx, p.ny, p.nz);
-            const AdjMom<R> m = adj_moments(fq, p);
-            for_q<0, 19>([&](auto qi) {
-                constexpr int q = decltype(qi)::value;
-                const R cu = cdot<q>(m.ux, m.uy, m.uz);
-                const R feq = wR<R>(q) * m.rho * (R(1) + R(3) * cu + R(4.5) * cu * cu - R(1.5) * m.uu);
-                fq[q] = fq[q] + p.omega * (feq - fq[q]);
-            });
+            const CellV<R> m = moments(fq, p.fx, p.fy, p.fz);
+            collide(fq, m, p.omega);
             const uint32_t lk = (fl & F_SPECIAL) ? p.links[id] : 0u;
             for_q<0, 19>([&](auto qi) {
                 constexpr int q = decltype(qi)::value;
@@ -183,7 +156,7 @@ __global__ void __launch_bounds__(256) adj_fwd(AdjP<R> p, const R* __restrict__ 
                     R v = fq[q];
                     if (cx(q) < 0 && c.x == 0) {
                         const R u = (R)uin[(int64_t)c.z * p.ny + c.y];
-                        v = wR<R>(q) * m.rho * (R(1) + R(3) * u + R(3) * u * u);
+                        v = wR<R>(q) * m.r * (R(1) + R(3) * u + R(3) * u * u);
                     } else if (cx(q) > 0 && c.x == p.nx - 1) {
                         v = fq[o];
                     } else if (cx(q) != 0 && drag_part && (p.flags[t] & F_OBST)) {
@@ -242,14 +215,14 @@ __global__ void __launch_bounds__(256) adj_bwd(AdjP<R> p, const R* __restrict__ 
     }
     AdjCell<IDX> c;
     c.init((uint32_t)id64, p.nx, p.ny, p.nz);
-    AdjMom<R> m;
+    CellV<R> m;
     {
         R fq[19];
         for_q<0, 19>([&](auto qi) {
             constexpr int q = decltype(qi)::value;
             fq[q] = f[(IDX)q * N + id];
         });
-        m = adj_moments(fq, p);
+        m = moments(fq, p.fx, p.fy, p.fz);
     }
     const uint32_t lk = (fl & F_SPECIAL) ? p.links[id] : 0u;
     R ls[19];
@@ -274,7 +247,7 @@ __global__ void __launch_bounds__(256) adj_bwd(AdjP<R> p, const R* __restrict__ 
                 if (cx(q) < 0 && c.x == 0) {
                     const R u = (R)uin[(int64_t)c.z * p.ny + c.y];
                     a_in += lo * wR<R>(q) * (R(1) + R(3) * u + R(3) * u * u);
-                    g_in += (double)(lo * wR<R>(q) * m.rho * (R(3) + R(6) * u));
+                    g_in += (double)(lo * wR<R>(q) * m.r * (R(3) + R(6) * u));
                     ls[q] = 0;
                 } else if (cx(q) > 0 && c.x == p.nx - 1) {
                     keep[o] = lo;
@@ -290,20 +263,28 @@ __global__ void __launch_bounds__(256) adj_bwd(AdjP<R> p, const R* __restrict__ 
         });
         if (c.x == 0 && g_uin) g_uin[(int64_t)c.z * p.ny + c.y] += g_in;
     }
-    R A = 0, Bx = 0, By = 0, Bz = 0;
-    for_q<0, 19>([&](auto qi) {
-        constexpr int q = decltype(qi)::value;
-        const R cu = cdot<q>(m.ux, m.uy, m.uz);
-        const R w = wR<R>(q);
-        A += ls[q] * w * (R(1) + R(3) * cu + R(4.5) * cu * cu - R(1.5) * m.uu);
-        const R t = ls[q] * w * m.rho;
-        const R k = R(3) + R(9) * cu;     // 3 + 9 c.u
-        Bx += t * plus_c<cx(q)>(-R(3) * m.ux, k);
-        By += t * plus_c<cy(q)>(-R(3) * m.uy, k);
-        Bz += t * plus_c<cz(q)>(-R(3) * m.uz, k);
+    // A and B per opposite pair (q, o), with S = w (ls_q + ls_o), D = w (ls_q - ls_o):
+    //   A = (1 - 1.5 u^2) sum S + sum c.u (4.5 c.u S + 3 D)
+    //   B = rho [sum c (9 c.u S + 3 D) - 3 u sum S]
+    const R uu = m.ux * m.ux + m.uy * m.uy + m.uz * m.uz;
+    R sw = wR<R>(0) * ls[0], A = 0, Bx = 0, By = 0, Bz = 0;
+    for_q<1, 19>([&](auto qi) {
+        constexpr int q = decltype(qi)::value, o = opp(q);
+        if constexpr (q < o) {
+            const R S = wR<R>(q) * (ls[q] + ls[o]), D = wR<R>(q) * (ls[q] - ls[o]);
+            const R cu = cdot<q>(m.ux, m.uy, m.uz);
+            const R e = R(4.5) * cu * S, k = e + R(3) * D;
+            sw += S;
+            A += cu * k;
+            Bx = plus_c<cx(q)>(Bx, e + k);
+            By = plus_c<cy(q)>(By, e + k);
+            Bz = plus_c<cz(q)>(Bz, e + k);
+        }
     });
+    A += (R(1) - R(1.5) * uu) * sw;
+    // (B carries rho, and the derivative of u divides by it)
+    const R gx = Bx - R(3) * m.ux * sw, gy = By - R(3) * m.uy * sw, gz = Bz - R(3) * m.uz * sw;
     const R om = p.omega;
-    const R gx = Bx / m.rho, gy = By / m.rho, gz = Bz / m.rho;
     const R base = om * (A - (gx * (m.ux - p.fx) + gy * (m.uy - p.fy) + gz * (m.uz - p.fz))) + a_in;
     for_q<0, 19>([&](auto qi) {
         constexpr int q = decltype(qi)::value;
