@@ -300,7 +300,8 @@ typedef struct lbm_adj_problem {
  * recomputed forward states).  host_mask: Nx*Ny*Nz bytes as lbm_set_solid_mask
  * takes them (walls 1|LBM_MASK_WALL are left out of the drag); u_inlet and
  * grad_inlet: Ny*Nz values, index z*Ny + y; u0 and grad_u0: three planes of
- * N values (u_x, u_y, u_z).  Synchronous; allocates its own device memory.  No
+ * N values (u_x, u_y, u_z); each of these four in host or device memory.
+ * Synchronous; allocates its own device memory.  No
  * reference counterpart (the reference has no inlet, drag or gradients). */
 int lbm_adjoint_run(const lbm_adj_problem* p, const uint8_t* host_mask, const double* u_inlet,
                     const double* u0, double* objective, double* grad_inlet, double* grad_u0);

@@ -171,6 +171,8 @@ def _sources_newer() -> bool:
 def lib():
     """Load (building it first if it is missing or stale) the CUDA library."""
     global _lib
+    if _lib is not None:      # (assigned once, complete)
+        return _lib
     with _lock:
         if _lib is None:
             if _sources_newer():

@@ -51,20 +51,27 @@ def objective(problem: DuctProblem, u_inlet, u0, precision: str = "f32", grad: b
     """J, or (J, dJ/du_inlet (nz, ny), dJ/du0 (3, nz, ny, nx)) when grad is set.
 
     u_inlet: (nz, ny) inlet x-velocity profile; u0: (3, nz, ny, nx) initial velocity."""
-    L = lib()
     nx, ny, nz = problem.nx, problem.ny, problem.nz
-    mask = np.ascontiguousarray(problem.mask, np.uint8)
     ui = np.ascontiguousarray(u_inlet, np.float64)
     u = np.ascontiguousarray(u0, np.float64)
-    if mask.size != nx * ny * nz or ui.size != ny * nz or u.size != 3 * nx * ny * nz:
+    if ui.size != ny * nz or u.size != 3 * nx * ny * nz:
+        raise ValueError("mask, u_inlet or u0 has the wrong size")
+    gi = np.empty((nz, ny), np.float64) if grad else None
+    gu = np.empty((3, nz, ny, nx), np.float64) if grad else None
+    J = _run(problem, precision, *[None if a is None else a.ctypes.data for a in (ui, u, gi, gu)])
+    return (J, gi, gu) if grad else J
+
+
+def _run(problem: DuctProblem, precision, ui, u0, gi, gu) -> float:
+    """lbm_adjoint_run on float64 arrays given by address, in host or device memory."""
+    mask = np.ascontiguousarray(problem.mask, np.uint8)
+    if mask.size != problem.nx * problem.ny * problem.nz:
         raise ValueError("mask, u_inlet or u0 has the wrong size")
     J = C.c_double(0.0)
-    gi = np.zeros((nz, ny), np.float64) if grad else None
-    gu = np.zeros((3, nz, ny, nx), np.float64) if grad else None
-    vp = lambda a: None if a is None else a.ctypes.data_as(C.c_void_p)
+    vp = lambda a: None if a is None else C.c_void_p(a)
     pc = problem._c(precision)
-    check(L.lbm_adjoint_run(C.byref(pc), vp(mask), vp(ui), vp(u), C.byref(J), vp(gi), vp(gu)))
-    return (J.value, gi, gu) if grad else J.value
+    check(lib().lbm_adjoint_run(C.byref(pc), mask.ctypes.data_as(C.c_void_p), vp(ui), vp(u0), C.byref(J), vp(gi), vp(gu)))
+    return J.value
 
 
 def _autograd_function():
@@ -75,6 +82,20 @@ def _autograd_function():
 
         @staticmethod
         def forward(ctx, u_inlet, u0, problem, precision="f32"):
+            here = torch.cuda.current_device() if u_inlet.is_cuda and u0.is_cuda else None
+            if here is not None and u_inlet.device.index == here and u0.device.index == here:
+                # the controls are where the library runs: no copies through the host
+                nx, ny, nz = problem.nx, problem.ny, problem.nz
+                ui, u = [t.detach().to(torch.float64).contiguous() for t in (u_inlet, u0)]
+                if ui.numel() != ny * nz or u.numel() != 3 * nx * ny * nz:
+                    raise ValueError("mask, u_inlet or u0 has the wrong size")
+                gi = torch.empty((nz, ny), dtype=torch.float64, device=u.device)
+                gu = torch.empty((3, nz, ny, nx), dtype=torch.float64, device=u.device)
+                # the library's own stream reads and writes them
+                torch.cuda.current_stream().synchronize()
+                J = _run(problem, precision, *[t.data_ptr() for t in (ui, u, gi, gu)])
+                ctx.save_for_backward(gi.to(u_inlet.dtype), gu.to(u0.dtype))
+                return torch.tensor(J, dtype=torch.float64, device=u_inlet.device)
             J, gi, gu = objective(problem, u_inlet.detach().cpu().numpy(), u0.detach().cpu().numpy(), precision,
                                   grad=True)
             ctx.save_for_backward(torch.from_numpy(gi).to(u_inlet.device, u_inlet.dtype),

@@ -107,9 +107,10 @@ def duct_sphere_mesh(nx: int, ny: int, nz: int, radius: float, center, levels: i
 
 def duct_mask(nx: int, ny: int, nz: int, obstacle: np.ndarray | None = None) -> np.ndarray:
     """Mask (nz, ny, nx) uint8: walls on the y and z faces (1|8), obstacle cells 1."""
-    m = np.zeros((nz, ny, nx), dtype=np.uint8)
-    if obstacle is not None:
-        m[obstacle.reshape(nz, ny, nx) != 0] = MASK_SOLID
+    if obstacle is None:
+        m = np.zeros((nz, ny, nx), dtype=np.uint8)
+    else:      # MASK_SOLID (1) where the obstacle is not 0: the comparison's own bytes
+        m = np.not_equal(obstacle.reshape(nz, ny, nx), 0, order="C").view(np.uint8)
     wall = MASK_SOLID | MASK_WALL
     m[:, 0, :] = wall
     m[:, ny - 1, :] = wall

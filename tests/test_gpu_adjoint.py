@@ -101,6 +101,27 @@ def test_ragged_grids_match_fp64_autodiff(gpu, dims, steps, window, every):
         assert np.linalg.norm(a - b) <= 1e-9 * np.linalg.norm(b)
 
 
+@pytest.mark.parametrize("dtype", ["float32", "float64"])
+def test_device_controls_equal_host_controls(gpu, tiny, dtype):
+    """Controls on the GPU, strided ones among them, take the path without host copies: the same bits."""
+    import torch
+    prob, ui, u0 = tiny
+    dt = getattr(torch, dtype)
+    out = []
+    for dev in ("cpu", "cuda"):
+        a = torch.tensor(ui.T.copy(), dtype=dt, device=dev).t().requires_grad_()
+        b = torch.tensor(u0, dtype=dt, device=dev).requires_grad_()
+        J = drag_objective(a, b, prob, "f64")
+        ga, gb = torch.autograd.grad(2.0 * J, (a, b))
+        assert J.device.type == dev and ga.dtype == dt and gb.dtype == dt
+        out.append((J.item(), ga.cpu().numpy(), gb.cpu().numpy()))
+    assert out[0][0] == out[1][0]
+    np.testing.assert_array_equal(out[0][1], out[1][1])
+    np.testing.assert_array_equal(out[0][2], out[1][2])
+    with pytest.raises(ValueError):
+        drag_objective(torch.zeros(3, 3, device="cuda"), torch.zeros(3, device="cuda"), prob)
+
+
 def test_adjoint_matches_central_differences(gpu):
     """A 64x32x32 copy of the adjoint case (sphere r=5 at (16,16,16)), 120 steps,
     drag averaged over steps 100-120: directional derivatives along random
