@@ -208,22 +208,27 @@ static int wait_pending_read(lbm_solver* s) {
 
 // Four plain steps as two two-step launches, f -> f2 -> f: the state ends in
 // the buffer it started from, so nothing outside the step sees the second one.
-static int enqueue_pairs(lbm_solver* s) {
+static int enqueue_pairs(lbm_solver* s, bool first) {
     const lbm::AAParams p = aa_params(s, false, false);
     float* f = static_cast<float*>(s->f);
     float* g = static_cast<float*>(s->f2);
-    const int zc = lbm::pair_zchunk(s->dom.nx, s->dom.ny, s->dom.nz, s->storage);
+    const int zc = lbm::pair_zchunk(s->dom.nx, s->dom.ny, s->dom.nz, s->storage, s->use_flags);
+    if (first) CK(lbm::launch_pair_solids(p, f, g, s->stream));
     CK(lbm::launch_aa_pair(p, f, g, zc, s->stream));
     CK(lbm::launch_aa_pair(p, g, f, zc, s->stream));
     return LBM_OK;
 }
 
 static int enqueue_steps(lbm_solver* s, int n) {
+    const bool pairs = is_aa(s) && !is_ref_push(s) && s->f2 && !s->zghost &&
+                       lbm::pair_zchunk(s->dom.nx, s->dom.ny, s->dom.nz, s->storage, s->use_flags) > 0;
+    bool first_pair = true;
     for (int i = 0; i < n; ++i) {
         // steps behind an odd parity and before one that writes macro fields or statistics
-        while (is_aa(s) && !is_ref_push(s) && s->f2 && !s->use_flags && !s->zghost && s->parity == 1 &&
+        while (pairs && s->parity == 1 &&
                n - i - (s->macro_out || s->stats_on ? 1 : 0) >= 4) {
-            const int rc = enqueue_pairs(s);
+            const int rc = enqueue_pairs(s, first_pair);
+            first_pair = false;
             if (rc != LBM_OK) return rc;
             i += 4;
         }
@@ -430,7 +435,7 @@ int lbm_create(const lbm_domain* dom, const lbm_options* opts, lbm_solver** out)
         return fail(LBM_ERR_CUDA);
     }
     // the second buffer of the two-step kernel; without it every step is a single one
-    if (is_aa(s) && !is_ref_push(s) && lbm::pair_zchunk(dom->nx, dom->ny, dom->nz, o.storage) > 0) {
+    if (is_aa(s) && !is_ref_push(s) && lbm::pair_zchunk(dom->nx, dom->ny, dom->nz, o.storage, false) > 0) {
         if (!dmalloc(&s->f2, s->esize * 19 * (size_t)N)) {
             cudaGetLastError();
             s->f2 = nullptr;

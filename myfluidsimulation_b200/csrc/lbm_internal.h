@@ -77,11 +77,14 @@ int64_t aa_odd_grid(int nx, int ny, int64_t planes, bool mask, int storage, Laun
 // One step of many instances in one persistent launch (FP32 populations, the
 // instances' flag bytes required); units: {instance, first, count, -} with
 // first/count in two-cell vectors (parity 0) or cells (parity 1).  stats != 0 writes NSTAT sums per unit into partials.
-// Two steps, an odd one and the even one behind it, from fa to fb (FP32, no solid
-// cells and no duct; parity 1 before and after, the whole grid, no macro fields or statistics).
+// Two steps, an odd one and the even one behind it, from fa to fb (FP32; parity 1
+// before and after, the whole grid, no macro fields or statistics; solid cells of fb
+// are left as they are).
 cudaError_t launch_aa_pair(const AAParams& p, const float* fa, float* fb, int zchunk, cudaStream_t s);
+// copies the solid cells' populations from fa to fb: before the first of those launches
+cudaError_t launch_pair_solids(const AAParams& p, const float* fa, float* fb, cudaStream_t s);
 // planes per block of that launch, or 0 where single steps are faster
-int pair_zchunk(int nx, int ny, int nz, int storage);
+int pair_zchunk(int nx, int ny, int nz, int storage, bool mask);
 // sets the dynamic shared-memory limit of its kernels (call outside graph capture)
 cudaError_t pair_prepare();
 cudaError_t launch_aa_batch(const AAParams* d_inst, const int4* d_units, int nunits, int parity, int stats,

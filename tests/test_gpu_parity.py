@@ -178,8 +178,8 @@ def test_reference_bounce_small_extents_vs_oracle(gpu, oracle, dims):
     assert vel_err(g["macros"][1:], mac[1:]) < TOL_F
 
 
-@pytest.mark.parametrize("dims", [(32, 8, 5), (33, 9, 7), (31, 7, 1), (64, 24, 49), (66, 17, 2), (3, 3, 3), (1, 1, 4),
-                                  (2, 40, 16), (100, 50, 6)])
+@pytest.mark.parametrize("dims", [(32, 8, 5), (31, 8, 1), (30, 8, 2), (63, 16, 3), (64, 24, 49), (61, 23, 9), (96, 15, 6),
+                                  (128, 7, 13)])
 @pytest.mark.parametrize("method", [METHOD_LEGACY, METHOD_HYBRID])
 def test_two_steps_at_a_time_equal_single_steps(gpu, method, dims):
     """Without solid cells a call of several steps takes them two at a time: same bits as one step per call, at
@@ -193,6 +193,36 @@ def test_two_steps_at_a_time_equal_single_steps(gpu, method, dims):
         for a, b in zip(many["macros"], one["macros"]):
             np.testing.assert_array_equal(a, b)
         assert many["stats"] == one["stats"]
+
+
+@pytest.mark.parametrize("dims,duct", [((193, 121, 120), False), ((254, 127, 88), False), ((224, 128, 97), True),
+                                       ((251, 96, 116), True)])
+@pytest.mark.parametrize("method", [METHOD_LEGACY, METHOD_HYBRID])
+def test_two_steps_at_a_time_equal_single_steps_with_solids(gpu, method, dims, duct):
+    """The same beyond L2 with solid cells scattered over tile edges and chunk ends, walls, a band, and a duct's inlet
+    and outlet at whole and partial tiles and odd widths; solid cells keep their populations."""
+    nx, ny, nz = dims
+    fields = init_fields(nx, ny, nz, seed=24)
+    mask = obstacle_mask(nx, ny, nz, seed=25, duct=duct)
+    got = []
+    for chunks in ([11], [1] * 11, [2, 9]):
+        s = Solver(nx, ny, nz, 0.6, (0, 0, 0) if duct else (1e-5, 2e-6, 0), method=method, bc=BC_DUCT if duct else BC_PERIODIC,
+                   inlet_u=0.04 if duct else 0.0)
+        s.set_solid_mask(mask)
+        if method == METHOD_HYBRID:
+            s.build_band(2)
+            s.set_shear_omega(1.3)
+        s.reinit_from_host(*fields)
+        s.enable_stats(True)
+        for c in chunks:
+            s.step(c)
+        got.append((s.state(), s.macros(), s.stats()))
+        s.close()
+    for st, mac, stats in got[1:]:
+        np.testing.assert_array_equal(st, got[0][0])
+        for a, b in zip(mac, got[0][1]):
+            np.testing.assert_array_equal(a, b)
+        assert stats == got[0][2]
 
 
 def test_hybrid_equals_legacy_by_default(gpu):
