@@ -94,15 +94,21 @@ __device__ __forceinline__ uint32_t cvt_rs_bf16x2(float lo, float hi, uint32_t r
 // Step kernels follow one another on a stream, and the small grids' steps take a few
 // microseconds each, of which the launch of the next one is a good part.  They are
 // launched so that a kernel may start while the one before it ends: its blocks take
-// the SMs that have gone idle and wait at step_begin() until everything before it has
-// completed and is visible.  Every kernel launched by launch_after() calls step_begin()
-// before its first access to global memory.  Measured, us per 50, 20 or 10 steps: the
-// 256x128x128 duct 5716 -> 5634 (Legacy) and 5974 -> 5837 (HOME, inlet), 201x93x77 F16
-// 969 -> 920, 128x128x96 with the reference's table 556 -> 537.  The batched step, one
-// persistent launch, lost 1 % with it and is launched plainly.
+// the SMs that have gone idle and wait at step_wait() until everything before it has
+// completed and is visible.  Every kernel launched by launch_after() calls step_wait()
+// before its first access to global memory, and step_next() lets the next kernel start
+// once every block has called it: at the top (step_begin) in the population steps, at the
+// end in the moment step, whose blocks lose 4-5 % on grids with a partial last wave when
+// the next step's blocks are already there (180x434x244 3.49 against 3.33 ms per 7 steps).
+// Measured, us per 50, 20 or 10 steps: the 256x128x128 duct 5716 -> 5634 (Legacy) and
+// 5971 -> 5870 (HOME, inlet), 201x93x77 F16 956 -> 918, 64^3 159 -> 136 (Legacy) and
+// 186 -> 179 (HOME), 128x128x96 with the reference's table 556 -> 537.  The batched step,
+// one persistent launch, lost 1 % with it and is launched plainly.
+__device__ __forceinline__ void step_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void step_next() { asm volatile("griddepcontrol.launch_dependents;"); }
 __device__ __forceinline__ void step_begin() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;");
+    step_wait();
+    step_next();
 }
 template <class... P, class... A>
 inline cudaError_t launch_after(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s, A&&... args) {

@@ -346,7 +346,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 8 ? 2 : 4) home_step(HomePara
     using E = typename HomeTypes<T>::E;
     using V = typename HomeTypes<T>::V;
     extern __shared__ __align__(16) unsigned char smraw[];
-    step_begin();
+    step_wait();
     E* sm = reinterpret_cast<E*>(smraw);
     const T* __restrict__ m = static_cast<const T*>(p.m);
     T* __restrict__ mn = static_cast<T*>(p.mn);
@@ -622,6 +622,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 8 ? 2 : 4) home_step(HomePara
         }
         __syncthreads();
     }
+    step_next();
     if constexpr (STATS) block_reduce_stats(acc, p.partials);
 }
 
