@@ -63,7 +63,9 @@ struct lbm_solver {
     int parity = 0;             // AA: 0 natural layout, 1 swapped; reference bounce: 0 A current, 1 B
     int64_t steps = 0;
     lbm::LaunchCfg cfg_even{0, 256}, cfg_odd{0, 256};
-    int home_zchunk = 16;
+    int home_zchunk = 16;       // planes per block: home_auto[flags in use], unless home_zchunk_set
+    int home_auto[2] = {16, 16};
+    bool home_zchunk_set = false;
     bool zghost = false;        // z-slab: planes 0 and nz-1 are ghosts, steps cover 1..nz-2
     uint32_t salt_base = 0;     // narrow stores: index of cell 0 in the whole grid
     // graph cache
@@ -138,6 +140,7 @@ int home_after_step(lbm_solver* s) {
 
 int rebuild_flags(lbm_solver* s) {
     s->use_flags = s->any_solid || s->bc == LBM_BC_DUCT || (s->method == LBM_METHOD_HYBRID && s->any_band);
+    if (!s->home_zchunk_set) s->home_zchunk = s->home_auto[s->use_flags];
     CK(lbm::launch_build_flags(s->any_solid ? s->mask : nullptr,
                                (s->method == LBM_METHOD_HYBRID && s->any_band) ? s->band : nullptr, s->flags,
                                s->links, s->dom.nx, s->dom.ny, s->dom.nz, s->bc == LBM_BC_DUCT, s->stream));
@@ -394,24 +397,20 @@ int lbm_create(const lbm_domain* dom, const lbm_options* opts, lbm_solver** out)
     const int sms = lbm::num_sms();
     s->cfg_even = {sms * 8, 256};
     s->cfg_odd = {sms * 12, 256};
-    // HOME: the longest z-chunk (fewest re-built halo planes) that still gives
-    // three waves of resident blocks, so the tail of the last wave stays short
+    // HOME: planes per block without and with flags (rebuild_flags takes the one that
+    // applies); the statistics partials have room for either
+    int home_blocks = 1;
     if (o.method == LBM_METHOD_HOME) {
         static const int bps = lbm::home_blocks_per_sm();
-        int zc = 4;
-        for (int c : {48, 32, 24, 16, 12, 10, 8, 6, 4}) {
-            if ((int64_t)lbm::home_num_blocks(dom->nx, dom->ny, dom->nz, std::min(c, dom->nz)) >=
-                (int64_t)sms * bps * 3) {
-                zc = c;
-                break;
-            }
+        for (int k = 0; k < 2; ++k) {
+            s->home_auto[k] = lbm::home_pick_zchunk(dom->nx, dom->ny, dom->nz, bps, k != 0);
+            home_blocks = std::max(home_blocks, lbm::home_num_blocks(dom->nx, dom->ny, dom->nz, s->home_auto[k]));
         }
-        s->home_zchunk = std::min(zc, dom->nz);
     }
     // the z-marching odd step's grid (solvers without a mask)
     const int64_t odd_blocks = lbm::aa_odd_blocks(dom->nx, dom->ny, dom->nz, o.storage, s->cfg_odd.threads);
     s->max_blocks = (int)std::max<int64_t>({s->cfg_even.blocks, s->cfg_odd.blocks, odd_blocks,
-                                            lbm::home_num_blocks(dom->nx, dom->ny, dom->nz, s->home_zchunk), 1});
+                                            home_blocks});
     auto dmalloc = [&](void** p, size_t b) { return cudaMalloc(p, b) == cudaSuccess; };
     bool ok = true;
     if (is_aa(s)) ok = ok && dmalloc(&s->f, s->esize * 19 * (size_t)N);
@@ -765,6 +764,7 @@ int lbm_set_home_zchunk(lbm_solver* s, int zchunk) {
         s->max_blocks = need;
     }
     s->home_zchunk = z;
+    s->home_zchunk_set = true;
     drop_graph(s);
     return LBM_OK;
 }

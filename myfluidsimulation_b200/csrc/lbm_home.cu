@@ -36,6 +36,7 @@
 //     cells of a pair in one conversion.
 // DRAM traffic is the 10 moments read once and written once (80 B per cell in
 // FP32, 40 B in F16/BF16) plus the halo re-reads that L2 does not absorb.
+#include <algorithm>
 #include <type_traits>
 
 #include "lbm_common.cuh"
@@ -700,6 +701,36 @@ cudaError_t home_prepare() {
 
 int home_num_blocks(int nx, int ny, int nz, int zchunk) {
     return ((nx + TX - 1) / TX) * ((ny + TY - 1) / TY) * ((nz + zchunk - 1) / zchunk);
+}
+
+// Planes per block of the moment step.  A block rebuilds zchunk + 2 planes, so long
+// chunks do less work and short ones leave more blocks.  The longest chunk that leaves
+// three waves of resident blocks is taken.  Where none does and there are neither solid
+// cells nor duct ends, it is that of 4, 6 and 8 planes with the least
+// a (waves + 1/4)(zchunk + 2) + b blocks (zchunk + 2), the measured time of a step in us
+// to about 8 % (96^3 22.2 -> 20.4 us with 6 planes for 4, 128x128x96 42.4 -> 37.6, 201x93x77
+// 52.0 -> 49.1); longer ones leave too little to even out the blocks.  A grid whose blocks fill half the slots or less takes
+// that chunk even if it is shorter (32^3 7.3 -> 3.9); above that a shorter one costs other
+// solvers on the device what it gains alone (three 64^3 solvers side by side: 5.2 us a step
+// each with 4 planes, 7.1 with 3).  Blocks at walls and duct ends take longer, and longer
+// chunks leave a long last wave (256x128x128 duct: 8 planes 116, 12 planes 113, 16 planes 130).
+int home_pick_zchunk(int nx, int ny, int nz, int blocks_per_sm, bool flags) {
+    const int64_t slots = (int64_t)num_sms() * blocks_per_sm;
+    int waves = 4;
+    for (int c : {48, 32, 24, 16, 12, 10, 8, 6})
+        if ((int64_t)home_num_blocks(nx, ny, nz, std::min(c, nz)) >= slots * 3) { waves = c; break; }
+    if (flags || waves > 4) return std::min(waves, nz);
+    int best = std::min(4, nz);
+    double least = 1e300;
+    for (int c : {1, 2, 4, 6, 8}) {
+        const int z = std::min(c, nz);
+        const int64_t tiles = home_num_blocks(nx, ny, 1, 1), chunks = (nz + z - 1) / z;
+        if (c < 4 && tiles * chunks > slots / 2) continue;
+        const double cost = 0.78 * ((double)((tiles * chunks + slots - 1) / slots) + 0.25) * (z + 2) +
+                            0.0027 * (double)(tiles * (nz + 2 * chunks));
+        if (cost < least) { least = cost; best = z; }
+    }
+    return best;
 }
 
 int home_blocks_per_sm() {

@@ -100,6 +100,8 @@ cudaError_t launch_aa_materialize(const AAParams& p, int storage, int parity, fl
 // sets the dynamic shared-memory limit of the HOME kernels (call outside graph capture)
 cudaError_t home_prepare();
 int home_num_blocks(int nx, int ny, int nz, int zchunk);
+// planes per block of the HOME step; flags: the grid has solid cells or duct ends
+int home_pick_zchunk(int nx, int ny, int nz, int blocks_per_sm, bool flags);
 // resident HOME blocks per SM (occupancy of the FP32 step kernel)
 int home_blocks_per_sm();
 cudaError_t launch_home_step(const HomeParams& p, int storage, int tile_y, int blocks_per_sm, cudaStream_t s);
