@@ -57,9 +57,16 @@ FORCE = (1e-5, 0.0, 0.0)
 DRAG_EVERY = 50
 RADIUS, CENTER = 16, (64, 64, 64)
 B0 = 2
-# algorithmic bytes per cell-update (state read once + written once, plus the mask/flag byte)
+# algorithmic bytes per cell of one pass (state read once + written once, plus the mask/flag byte)
 BYTES = {"legacy": 19 * 4 * 2 + 1, "hybrid": 19 * 4 * 2 + 1, "home": 10 * 4 * 2 + 1}
-KERNEL = {"legacy": "aa_even/aa_odd", "hybrid": "aa_even/aa_odd", "home": "home_step"}
+KERNEL = {"legacy": "aa_pair", "hybrid": "aa_pair", "home": "home_step"}
+# LBM step kernels of one 50-step interval.  On the duct Legacy/Hybrid take the first step and the
+# one with the statistics singly, and the 48 between them two at a time (aa_pair), each pass one read and one
+# write of the state; HOME takes every step singly.
+PASSES = {"legacy": {"aa_even": 1, "aa_pair": 24, "aa_odd": 1}, "home": {"home_step": DRAG_EVERY}}
+PASSES["hybrid"] = PASSES["legacy"]
+# plus the statistics' final pass and, for Legacy/Hybrid, pair_solids (copies what solid cells hold) once
+LAUNCHES = {"legacy": 26 + 2, "hybrid": 26 + 2, "home": DRAG_EVERY + 1}
 METRIC = "D3Q19 MLUPS (Legacy BGK FP32, duct 256x128x128 past a voxelized sphere)"
 WORKLOAD_TEXT = {
     "periodic": "duct 256x128x128, y/z walls as solid cells, icosphere (5120 triangles, r=16, centre (64,64,64)) "
@@ -193,13 +200,13 @@ def make_solver(method, workload, mask, stream):
 
 
 def kernel_split(s, method, torch, launches=40):
-    """Per-kernel device time, summing to the time of back-to-back steps.
+    """Device time per launch of each step kernel, launched back to back.
 
-    The total is ONE lbm_step(launches) call (no macro fields, no statistics)
-    between two CUDA events, so nothing sits between the launches.  For the AA
-    methods the even/odd shares come from a second pass of single-step
-    launches with a CUDA event between every two (no synchronisation inside
-    the loop), whose median intervals split that total.  Returns
+    HOME: one lbm_step(launches) call between two CUDA events.  AA methods: the
+    same over single-step calls, split into even and odd by a second pass with a
+    CUDA event between every two (no synchronisation inside the loop); then one
+    call of 2 x launches steps from an odd parity, which is `launches` passes of
+    aa_pair (and one pair_solids).  No macro fields, no statistics.  Returns
     {kernel: us per launch}."""
     st = torch.cuda.current_stream()
     s.enable_stats(False)
@@ -208,7 +215,11 @@ def kernel_split(s, method, torch, launches=40):
     e0 = torch.cuda.Event(enable_timing=True)
     e1 = torch.cuda.Event(enable_timing=True)
     e0.record(st)
-    s.step(launches)                   # an even count: as many even as odd launches
+    if method == "home":
+        s.step(launches)
+    else:
+        for _ in range(launches):      # an even count: as many even as odd launches
+            s.step(1)
     e1.record(st)
     torch.cuda.synchronize()
     mean_us = 1e3 * e0.elapsed_time(e1) / launches
@@ -224,11 +235,20 @@ def kernel_split(s, method, torch, launches=40):
         ev[i + 1].record(st)
     torch.cuda.synchronize()
     t = [1e3 * ev[i].elapsed_time(ev[i + 1]) for i in range(launches)]
+    if s.steps % 2 == 0:
+        s.step(1)
+    e0.record(st)
+    s.step(2 * launches)               # a multiple of four
+    e1.record(st)
+    torch.cuda.synchronize()
+    pair_us = 1e3 * e0.elapsed_time(e1) / launches
+    s.step(1)                          # back to an even parity
     s.set_macro_output(True)
     s.enable_stats(True)
     a, b = statistics.median(t[0::2]), statistics.median(t[1::2])
     names = ("aa_even", "aa_odd") if par == 0 else ("aa_odd", "aa_even")
-    return {names[0]: round(2 * mean_us * a / (a + b), 2), names[1]: round(2 * mean_us * b / (a + b), 2)}
+    return {names[0]: round(2 * mean_us * a / (a + b), 2), names[1]: round(2 * mean_us * b / (a + b), 2),
+            "aa_pair": round(pair_us, 2)}
 
 
 def run_method(method, workload, mask, args, torch, dist=None):
@@ -251,7 +271,7 @@ def run_method(method, workload, mask, args, torch, dist=None):
         dist.barrier()
     ms = e0.elapsed_time(e1)
     st_ = s.stats()
-    res = {"ms_total": ms, "launches": args.steps * (DRAG_EVERY + 1), "band_cells": nb,
+    res = {"ms_total": ms, "launches": args.steps * LAUNCHES[method], "band_cells": nb,
            "drag_last": [st_["drag_x"], st_["drag_y"], st_["drag_z"]], "mass": st_["mass"],
            "kernel_us": kernel_split(s, method, torch)}
     return s, res
@@ -444,8 +464,8 @@ def precision_study(args, torch):
     """512^3 periodic Taylor-Green vortex (tau 0.51, u0 0.05, k 2pi/512), Legacy and
     HOME, in FP64 (storage and arithmetic: the reference form), FP32, F16 and BF16:
       * MLUPS over --steps steps after 4 warm-up steps (CUDA events, macro output
-        off), with the roofline fraction of the algorithmic bytes, and the
-        even/odd launch split (events between back-to-back launches);
+        off), the even/odd split of single-step launches (events between
+        back-to-back launches), and their roofline fraction of the algorithmic bytes;
       * from the initial field, the kinetic energy (FP64 reduction on the GPU)
         every --tgv-every steps up to --tgv-steps, and the fields at the end;
       * every form's energy curve (max relative error over the samples) and
@@ -504,8 +524,10 @@ def precision_study(args, torch):
             s.synchronize()
             fields = [_device_field(p_, N, torch) for p_ in s.macro_ptrs()]
             b = ncomp * esz * 2
+            # of the single-step launches: FP32 Legacy takes two steps per pass in one call
+            single_us = 0.5 * (statistics.median(t[0::2]) + statistics.median(t[1::2]))
             res = {"mlups": round(mlups, 1), "us_per_step": round(ms * 1e3 / args.steps, 1),
-                   "roofline_frac": round(N * b / (ms * 1e-3 / args.steps) / 1e9 / peak, 4), "bytes_per_cell": b,
+                   "roofline_frac": round(N * b / (single_us * 1e-6) / 1e9 / peak, 4), "bytes_per_cell": b,
                    "us_launch_a_b": [round(statistics.median(t[0::2]), 1), round(statistics.median(t[1::2]), 1)],
                    "ke_final_over_initial": curve[-1] / (curve[0] if curve else 1.0)}
             if sto == STORE_F64:
@@ -1179,12 +1201,13 @@ def main():
         m, w = keys[args.profile]
         s, _ = make_solver(m, w, mask, st.cuda_stream)
         s.enable_stats(False)
-        s.set_macro_output(False)      # the plain launches that make up 49 of every 50 bench steps
+        s.set_macro_output(False)      # the plain launches of the bench's steps
         for _ in range(4):
             s.step(1)
+        s.step(9)                      # Legacy/Hybrid: one single step, then four passes of aa_pair
         s.synchronize()
         s.close()
-        print(json.dumps({"profile": args.profile, "steps": 4}))
+        print(json.dumps({"profile": args.profile, "steps": 13}))
         return
     runs = [k for k in args.methods.split(",") if k]
     for k in runs:
@@ -1207,18 +1230,20 @@ def main():
         ms = float(ms.item())
         cell_updates = N * DRAG_EVERY * args.steps * world
         mlups = cell_updates / (ms * 1e-3) / 1e6
-        per_launch_ms = r["ms_total"] / (DRAG_EVERY * args.steps)
-        achieved = N * BYTES[mth] / (per_launch_ms * 1e-3) / 1e9
+        passes = sum(PASSES[mth].values())
+        per_pass_ms = r["ms_total"] / (passes * args.steps)
+        achieved = N * BYTES[mth] / (per_pass_ms * 1e-3) / 1e9
         tr = profile_traffic(mth)
         ku = r["kernel_us"]
-        split_ms = DRAG_EVERY * sum(ku.values()) / len(ku) / 1e3
+        split_ms = sum(n * ku[k] for k, n in PASSES[mth].items()) / 1e3
         results[key] = {"mlups": round(mlups, 1), "ms_per_step": round(ms / args.steps, 4),
                         "workload": wl, "kernel_us": ku,
                         "kernel_split_ms_per_step": round(split_ms, 4),
                         "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                                      "frac": round(achieved / peak, 4),
                                      "traffic": None if tr is None else int(round(tr * N)),
-                                     "kernel": KERNEL[mth], "bytes_per_cell": BYTES[mth]},
+                                     "kernel": KERNEL[mth], "bytes_per_cell": BYTES[mth],
+                                     "passes_per_50_steps": passes},
                         "kernel_frac": {k: round(N * BYTES[mth] / (v * 1e-6) / 1e9 / peak, 4) for k, v in ku.items()},
                         "drag": [round(x, 6) for x in r["drag_last"]], "mass": round(r["mass"], 3),
                         "launches": r["launches"]}
@@ -1268,7 +1293,7 @@ def main():
             "value": h["mlups"], "unit": "MLUPS", "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
             "ms_per_step": h["ms_per_step"], "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
             "dtype": "f32", "data": "synthetic", "config": config,
-            "bounce": "halfway bounce-back, AA pattern in place",
+            "bounce": "halfway bounce-back, AA pattern",
             "roofline": dict(h["roofline"], peak_kind=peak_kind),
             "e2e": {"value": round(e2e_mlups, 1), "unit": "MLUPS", "h2d_bytes_per_step": h2d,
                     "d2h_bytes_per_step": d2h, "wall_ms": round(e2e_wall, 2)},

@@ -2,7 +2,8 @@
 //
 // One lbm_solver replaces the reference's three classes (src/lbm/lbm3d_legacy.hpp,
 // lbm3d_home.hpp, lbm3d_hybrid.hpp).  Memory per cell:
-//   Legacy/Hybrid: one population buffer (AA pattern), 19 x 4 B (F32) or 19 x 2 B
+//   Legacy/Hybrid: one population buffer (AA pattern; F32 with halfway bounce-back a
+//                  second one for two steps per pass), 19 x 4 B (F32) or 19 x 2 B
 //                  (F16/BF16), plus rho,u,v,w (16 B), mask, flags (1 B each) and a
 //                  link word (4 B); the reference holds two population buffers.
 //   HOME:          two moment buffers of 10 x 4 B (or 10 x 2 B), as the reference.
@@ -41,7 +42,7 @@ struct lbm_solver {
     size_t esize = 4;
 
     void* f = nullptr;          // AA populations (reference bounce: buffer A)
-    void* f2 = nullptr;         // reference bounce only: buffer B
+    void* f2 = nullptr;         // reference bounce: buffer B; F32 halfway: two-step passes (may be null)
     void* m[2] = {nullptr, nullptr};   // HOME moments
     int cur = 0;
     float* macro = nullptr;     // 4*N floats: rho, ux, uy, uz (AA; HOME F16/BF16 export)
