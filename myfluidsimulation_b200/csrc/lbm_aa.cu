@@ -610,6 +610,15 @@ int64_t aa_odd_grid(int nx, int ny, int64_t planes, bool mask, int storage, Laun
     return (int64_t)std::max(1, cfg.blocks / segs) * segs;
 }
 
+int64_t aa_stat_blocks(int nx, int ny, int nz, int storage, LaunchCfg even, LaunchCfg odd) {
+    int64_t most = even.blocks;
+    for (int ghosts : {0, 2})
+        if (nz > ghosts)
+            for (bool mask : {false, true})
+                most = std::max(most, aa_odd_grid(nx, ny, nz - ghosts, mask, storage, odd));
+    return most;
+}
+
 namespace {
 
 template <class ST, int MODE, class IDX>

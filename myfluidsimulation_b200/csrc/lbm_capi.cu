@@ -60,7 +60,6 @@ struct lbm_solver {
     bool any_band = false;
     bool stats_on = false;
     bool macro_out = true;      // write rho,u on the last substep of each lbm_step
-    int last_stat_blocks = 0;
     int parity = 0;             // AA: 0 natural layout, 1 swapped; reference bounce: 0 A current, 1 B
     int64_t steps = 0;
     lbm::LaunchCfg cfg_even{0, 256}, cfg_odd{0, 256};
@@ -108,8 +107,16 @@ void drop_graph(lbm_solver* s) {
     s->g_sub = 0; s->g_parity = -1; s->g_stats = -1;
 }
 
-// planes a HOME step covers (a z-slab skips its two ghost planes)
-int home_planes(const lbm_solver* s) { return s->zghost ? s->dom.nz - 2 : s->dom.nz; }
+// planes a step covers (a z-slab skips its two ghost planes)
+int own_planes(const lbm_solver* s) { return s->zghost ? s->dom.nz - 2 : s->dom.nz; }
+
+// blocks of the next step's launch, one statistics partial each
+int64_t next_stat_blocks(const lbm_solver* s) {
+    if (!is_aa(s)) return lbm::home_num_blocks(s->dom.nx, s->dom.ny, own_planes(s), s->home_zchunk);
+    if (is_ref_push(s)) return s->cfg_odd.blocks;
+    if (s->parity == 0) return s->cfg_even.blocks;
+    return lbm::aa_odd_grid(s->dom.nx, s->dom.ny, own_planes(s), s->use_flags, s->storage, s->cfg_odd);
+}
 
 float* home_macro_base(lbm_solver* s) {
     // F32 HOME exposes its state directly (d_rho() = m + 0*N, home.cu:355-362)
@@ -245,28 +252,26 @@ static int enqueue_steps(lbm_solver* s, int n) {
             const int rc = wait_pending_read(s);
             if (rc != LBM_OK) return rc;
         }
+        const int64_t stat_blocks = st ? next_stat_blocks(s) : 0;
+        if (stat_blocks > s->max_blocks) {
+            set_error("lbm_step: more blocks than statistics partials");
+            return LBM_ERR_SIZE;
+        }
         if (is_ref_push(s)) {
             lbm::AAParams p = aa_params(s, mac, st);
             CK(lbm::launch_ref_push(p, static_cast<const float*>(cur_pop(s)), static_cast<float*>(other_pop(s)),
                                     s->cfg_odd, s->stream));
             s->parity ^= 1;
-            if (st) s->last_stat_blocks = s->cfg_odd.blocks;
         } else if (is_aa(s)) {
             lbm::AAParams p = aa_params(s, mac, st);
-            const lbm::LaunchCfg cfg = s->parity == 0 ? s->cfg_even : s->cfg_odd;
-            CK(lbm::launch_aa_step(p, s->storage, s->parity, cfg, s->stream));
-            if (st)
-                s->last_stat_blocks = s->parity == 0 ? cfg.blocks
-                                                     : (int)lbm::aa_odd_grid(p.nx, p.ny, p.cells / ((int64_t)p.nx * p.ny),
-                                                                             p.flags != nullptr, s->storage, cfg);
+            CK(lbm::launch_aa_step(p, s->storage, s->parity, s->parity == 0 ? s->cfg_even : s->cfg_odd, s->stream));
             s->parity ^= 1;
         } else {
             lbm::HomeParams p = home_params(s, st);
             CK(lbm::launch_home_step(p, s->storage, 8, 3, s->stream));
             s->cur ^= 1;
-            if (st) s->last_stat_blocks = lbm::home_num_blocks(s->dom.nx, s->dom.ny, home_planes(s), s->home_zchunk);
         }
-        if (st) CK(lbm::launch_finalize_stats(s->partials, s->last_stat_blocks, s->stats, s->stream));
+        if (st) CK(lbm::launch_finalize_stats(s->partials, (int)stat_blocks, s->stats, s->stream));
     }
     if (n > 0) {
         const int rc = home_after_step(s);
@@ -398,20 +403,18 @@ int lbm_create(const lbm_domain* dom, const lbm_options* opts, lbm_solver** out)
     const int sms = lbm::num_sms();
     s->cfg_even = {sms * 8, 256};
     s->cfg_odd = {sms * 12, 256};
-    // HOME: planes per block without and with flags (rebuild_flags takes the one that
-    // applies); the statistics partials have room for either
-    int home_blocks = 1;
-    if (o.method == LBM_METHOD_HOME) {
+    // statistics partials: room for every launch that a step of this solver can be
+    if (is_aa(s)) {
+        s->max_blocks = (int)std::max<int64_t>(
+            s->cfg_odd.blocks, lbm::aa_stat_blocks(dom->nx, dom->ny, dom->nz, o.storage, s->cfg_even, s->cfg_odd));
+    } else {
+        // planes per block without and with flags (rebuild_flags takes the one that applies)
         static const int bps = lbm::home_blocks_per_sm();
         for (int k = 0; k < 2; ++k) {
             s->home_auto[k] = lbm::home_pick_zchunk(dom->nx, dom->ny, dom->nz, bps, k != 0);
-            home_blocks = std::max(home_blocks, lbm::home_num_blocks(dom->nx, dom->ny, dom->nz, s->home_auto[k]));
+            s->max_blocks = std::max(s->max_blocks, lbm::home_num_blocks(dom->nx, dom->ny, dom->nz, s->home_auto[k]));
         }
     }
-    // the z-marching odd step's grid (solvers without a mask)
-    const int64_t odd_blocks = lbm::aa_odd_blocks(dom->nx, dom->ny, dom->nz, o.storage, s->cfg_odd.threads);
-    s->max_blocks = (int)std::max<int64_t>({s->cfg_even.blocks, s->cfg_odd.blocks, odd_blocks,
-                                            home_blocks});
     auto dmalloc = [&](void** p, size_t b) { return cudaMalloc(p, b) == cudaSuccess; };
     bool ok = true;
     if (is_aa(s)) ok = ok && dmalloc(&s->f, s->esize * 19 * (size_t)N);
@@ -751,7 +754,7 @@ int lbm_set_home_zchunk(lbm_solver* s, int zchunk) {
     if (s->method != LBM_METHOD_HOME) { set_error("lbm_set_home_zchunk: HOME only"); return LBM_ERR_INVALID; }
     if (zchunk < 1) { set_error("lbm_set_home_zchunk: zchunk must be >= 1"); return LBM_ERR_INVALID; }
     const int z = std::min(zchunk, s->dom.nz);
-    const int need = lbm::home_num_blocks(s->dom.nx, s->dom.ny, home_planes(s), z);
+    const int need = lbm::home_num_blocks(s->dom.nx, s->dom.ny, s->dom.nz, z);      // (ghost planes can be switched off later)
     if (need > s->max_blocks) {
         // per-block statistics partials: grow once the step queue has drained
         CK(cudaStreamSynchronize(s->stream));

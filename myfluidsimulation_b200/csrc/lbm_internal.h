@@ -74,6 +74,10 @@ int64_t aa_odd_blocks(int nx, int ny, int64_t planes, int storage, int threads);
 // cfg.blocks rounded down to a multiple of the row segments (a 2-D grid of
 // rows x segments)
 int64_t aa_odd_grid(int nx, int ny, int64_t planes, bool mask, int storage, LaunchCfg cfg);
+// most blocks, one statistics partial each, that a step of either parity launches, with or
+// without a mask, on the whole grid or as a z-slab of nz - 2 planes of its own.  (Fewer planes
+// can give more blocks: a shorter run of planes per block is chosen for them.)
+int64_t aa_stat_blocks(int nx, int ny, int nz, int storage, LaunchCfg even, LaunchCfg odd);
 // One step of many instances in one persistent launch (FP32 populations, the
 // instances' flag bytes required); units: {instance, first, count, -} with
 // first/count in two-cell vectors (parity 0) or cells (parity 1).  stats != 0 writes NSTAT sums per unit into partials.

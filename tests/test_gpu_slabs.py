@@ -277,3 +277,26 @@ def test_plan_exchange_equals_pairwise_and_graph_replay(gpu):
             sl.close()
     np.testing.assert_array_equal(runs[0], runs[1])
     np.testing.assert_array_equal(runs[0], runs[2])
+
+
+@pytest.mark.parametrize("method", [METHOD_LEGACY, METHOD_HOME])
+def test_statistics_of_large_slabs_without_a_mask(gpu, method):
+    """Slabs of 165 planes and two ghost planes: the odd step has 5312 blocks of two planes each, more than the
+    3584 blocks of three that the same grid's odd step has without ghost planes."""
+    dims = (64, 256, 330)
+    f = fields(*dims, seed=6)
+    kw = dict(force=(1e-5, 2e-6, 0.0), method=method)
+    one, sl = Solver(*dims, 0.58, **kw), SlabSet(*dims, 0.58, 2, **kw)
+    for obj in (one, sl):
+        obj.reinit_from_host(*f)
+        obj.enable_stats(True)
+    for n in (2, 1):      # the last step an odd one, then an even one
+        for obj in (one, sl):
+            obj.step(n)
+            obj.synchronize()
+        s1, s2 = one.stats(), sl.stats()
+        scale = max(abs(v) for v in s1.values())
+        for k in s1:
+            assert s2[k] == pytest.approx(s1[k], rel=1e-12, abs=1e-12 * scale), k
+    one.close()
+    sl.close()
