@@ -264,27 +264,41 @@ __global__ void __launch_bounds__(256) adj_bwd(AdjP<R> p, const R* __restrict__ 
         });
         if (c.x == 0 && g_uin) g_uin[(int64_t)c.z * p.ny + c.y] += g_in;
     }
-    // A and B per opposite pair (q, o), with S = w (ls_q + ls_o), D = w (ls_q - ls_o):
-    //   A = (1 - 1.5 u^2) sum S + sum c.u (4.5 c.u S + 3 D)
-    //   B = rho [sum c (9 c.u S + 3 D) - 3 u sum S]
-    const R uu = m.ux * m.ux + m.uy * m.uy + m.uz * m.uz;
-    R sw = wR<R>(0) * ls[0], A = 0, Bx = 0, By = 0, Bz = 0;
-    for_q<1, 19>([&](auto qi) {
-        constexpr int q = decltype(qi)::value, o = opp(q);
-        if constexpr (q < o) {
-            const R S = wR<R>(q) * (ls[q] + ls[o]), D = wR<R>(q) * (ls[q] - ls[o]);
-            const R cu = cdot<q>(m.ux, m.uy, m.uz);
-            const R e = R(4.5) * cu * S, k = e + R(3) * D;
-            sw += S;
-            A += cu * k;
-            Bx = plus_c<cx(q)>(Bx, e + k);
-            By = plus_c<cy(q)>(By, e + k);
-            Bz = plus_c<cz(q)>(Bz, e + k);
-        }
-    });
-    A += (R(1) - R(1.5) * uu) * sw;
-    // (B carries rho, and the derivative of u divides by it)
-    const R gx = Bx - R(3) * m.ux * sw, gy = By - R(3) * m.uy * sw, gz = Bz - R(3) * m.uz * sw;
+    // A and B from sums over the opposite pairs (q, o) of one weight w, with
+    // S = ls_q + ls_o, D = ls_q - ls_o:
+    //   A = sum w [(1 - 1.5 u^2) sum S + sum c.u (4.5 c.u S + 3 D)]
+    //   B = rho sum w [sum c (9 c.u S + 3 D) - 3 u sum S]
+    // The weights are multiplied in once per sum, their own rounding compensated (mulk), as
+    // the forward step does: sum w_q of the rounded weights is 1.5e-8 too large, a bias of
+    // omega times that per step, 2.7e-6 over 100 steps at tau 0.56.  dJ/du0 of 48x32x32 after
+    // 100 steps is off by 4.4e-7 (2-norm, relative to FP64), by 2.5e-6 with rounded weights.
+    // (B carries rho, and the derivative of u divides by it.)
+    const R iso = R(1) - R(1.5) * (m.ux * m.ux + m.uy * m.uy + m.uz * m.uz);
+    const R l0 = mulk(ls[0], K3_HI, K3_LO), n0 = R(-3) * l0;
+    R A = iso * l0, gx = m.ux * n0, gy = m.uy * n0, gz = m.uz * n0;
+    auto add_pairs = [&](auto q0, auto q1, float hi, float lo) {
+        R s = 0, a = 0, bx = 0, by = 0, bz = 0;
+        for_q<decltype(q0)::value, decltype(q1)::value>([&](auto qi) {
+            constexpr int q = decltype(qi)::value, o = opp(q);
+            if constexpr (q < o) {
+                const R S = ls[q] + ls[o], D = ls[q] - ls[o];
+                const R cu = cdot<q>(m.ux, m.uy, m.uz);
+                const R e = R(4.5) * cu * S, k = e + R(3) * D;
+                s += S;
+                a += cu * k;
+                bx = plus_c<cx(q)>(bx, e + k);
+                by = plus_c<cy(q)>(by, e + k);
+                bz = plus_c<cz(q)>(bz, e + k);
+            }
+        });
+        const R s3 = R(3) * s;
+        A += mulk(a + iso * s, hi, lo);
+        gx += mulk(bx - m.ux * s3, hi, lo);
+        gy += mulk(by - m.uy * s3, hi, lo);
+        gz += mulk(bz - m.uz * s3, hi, lo);
+    };
+    add_pairs(QC<1>{}, QC<7>{}, K18_HI, K18_LO);
+    add_pairs(QC<7>{}, QC<19>{}, K36_HI, K36_LO);
     const R om = p.omega;
     const R base = om * (A - (gx * (m.ux - p.fx) + gy * (m.uy - p.fy) + gz * (m.uz - p.fz))) + a_in;
     for_q<0, 19>([&](auto qi) {

@@ -122,6 +122,19 @@ def test_device_controls_equal_host_controls(gpu, tiny, dtype):
         drag_objective(torch.zeros(3, 3, device="cuda"), torch.zeros(3, device="cuda"), prob)
 
 
+@pytest.mark.parametrize("seed", [1, 2])
+def test_fp32_gradient_carries_no_bias_of_the_weights(gpu, seed):
+    """The FP32 weights add up to 1 + 1.5e-8 (their own rounding): taken as they are, each reverse step adds a relative
+    error of 1.5e-8 / tau, of one sign, to the adjoint field.  Half of what 100 steps add up to is the bound."""
+    nx, ny, nz, tau, steps = 48, 32, 32, 0.56, 100
+    prob = DuctProblem(nx, ny, nz, tau, duct(nx, ny, nz, 4.8, (12, 16, 16)), n_steps=steps, window=(91, 100),
+                       checkpoint_every=25)
+    ui, u0 = [np.float32(a) for a in controls(nx, ny, nz, seed)]
+    _, gi64, gu64 = objective(prob, ui, u0, "f64", grad=True)
+    _, gi32, gu32 = objective(prob, ui, u0, "f32", grad=True)
+    assert np.linalg.norm(gu32 - gu64) < 0.5 * steps * 1.5e-8 / tau * np.linalg.norm(gu64)
+
+
 def test_adjoint_matches_central_differences(gpu):
     """A 64x32x32 copy of the adjoint case (sphere r=5 at (16,16,16)), 120 steps,
     drag averaged over steps 100-120: directional derivatives along random
