@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(256) adj_fwd(AdjP<R> p, const R* __restrict__ 
         } else {
             AdjCell<IDX> c;
             c.init((uint32_t)id64, p.nx, p.ny, p.nz);
-            const CellV<R> m = moments(fq, p.fx, p.fy, p.fz);
+            const CellV<R> m = moments<false>(fq, p.fx, p.fy, p.fz);   // u = j / rho + F whatever the sign of rho
             collide(fq, m, p.omega);
             const uint32_t lk = (fl & F_SPECIAL) ? p.links[id] : 0u;
             for_q<0, 19>([&](auto qi) {
@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(256) adj_bwd(AdjP<R> p, const R* __restrict__ 
             constexpr int q = decltype(qi)::value;
             fq[q] = f[(IDX)q * N + id];
         });
-        m = moments(fq, p.fx, p.fy, p.fz);
+        m = moments<false>(fq, p.fx, p.fy, p.fz);
     }
     const uint32_t lk = (fl & F_SPECIAL) ? p.links[id] : 0u;
     R ls[19];

@@ -65,6 +65,9 @@ __device__ __forceinline__ D2 vrcp_pos(D2 r) { return {r.x > 0.0 ? 1.0 / r.x : 0
 // scalar reciprocal with the same rule
 __device__ __forceinline__ float vrcp_pos(float r) { return r > 0.f ? __frcp_rn(r) : 0.f; }
 __device__ __forceinline__ double vrcp_pos(double r) { return r > 0.0 ? 1.0 / r : 0.0; }
+// and without it
+__device__ __forceinline__ float vrcp(float r) { return __frcp_rn(r); }
+__device__ __forceinline__ double vrcp(double r) { return 1.0 / r; }
 
 // ---- BGK on one cell (V = float, double) or two (V = float2, D2) -----------
 template <class V>
@@ -74,7 +77,9 @@ struct CellV {
 
 // Pre-collision moments with the velocity-shift force (legacy.cu:78-90).
 // Opposite pairs are summed first: s = f_q + f_opp, d = f_q - f_opp.
-template <class V, class R>
+// EMPTY: u = F where rho is not positive, as in the solvers; otherwise u = j / rho + F
+// there too, which is what the adjoint differentiates (one cell only).
+template <bool EMPTY = true, class V, class R>
 __device__ __forceinline__ CellV<V> moments(const V (&f)[19], R fx, R fy, R fz) {
     // pairs with their positive member: (1,2) x, (3,4) y, (5,6) z, (7,10) +x+y,
     // (9,8) +x-y, (11,14) +x+z, (13,12) +x-z, (15,18) +y+z, (17,16) +y-z
@@ -92,7 +97,10 @@ __device__ __forceinline__ CellV<V> moments(const V (&f)[19], R fx, R fy, R fz) 
     const V jx = vadd(vadd(vadd(d12, d7), vadd(d9, d11)), d13);
     const V jy = vadd(vsub(vadd(d34, d7), d9), vadd(d15, d17));
     const V jz = vadd(vsub(vadd(d56, d11), d13), vsub(d15, d17));
-    const V inv = vrcp_pos(c.r);
+    V inv = vrcp_pos(c.r);
+    // (behind a test: taken unconditionally it costs the adjoint's reverse step 80 registers for 64)
+    if constexpr (!EMPTY)
+        if (!(c.r > V(0))) inv = vrcp(c.r);
     c.ux = vfma(jx, inv, vsplat(fx, V{}));
     c.uy = vfma(jy, inv, vsplat(fy, V{}));
     c.uz = vfma(jz, inv, vsplat(fz, V{}));

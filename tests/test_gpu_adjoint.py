@@ -135,6 +135,31 @@ def test_fp32_gradient_carries_no_bias_of_the_weights(gpu, seed):
     assert np.linalg.norm(gu32 - gu64) < 0.5 * steps * 1.5e-8 / tau * np.linalg.norm(gu64)
 
 
+@pytest.mark.parametrize("seed", [0, 3, 6])
+def test_negative_densities_match_fp64_autodiff(gpu, seed):
+    """Velocities of order one leave negative densities behind the first step: u = j / rho there too, in the step and in
+    what the reverse step differentiates.  A relative change of 1e-15 in u0 moves J and the gradients by up to 1e-12."""
+    import torch
+    from torch_duct import TorchDuct
+    nx, ny, nz, steps = 12, 7, 9, 3
+    rng = np.random.default_rng(seed)
+    mask = (rng.random((nz, ny, nx)) < 0.1).astype(np.uint8)
+    mask[0] = W.MASK_SOLID | W.MASK_WALL
+    u0 = rng.uniform(-1, 1, (3, nz, ny, nx))
+    ui = 0.04 + 0.005 * rng.standard_normal((nz, ny))
+    td = TorchDuct(mask, 0.8)
+    tui, tu0 = torch.tensor(ui, requires_grad=True), torch.tensor(u0, requires_grad=True)
+    f = td.step(td.init(tu0.detach()), tui.detach())[0]
+    assert (f.sum(0)[~td.solid] < 0).sum() > 5
+    Jt = td.objective(tui, tu0, steps, (1, steps))
+    Jt.backward()
+    prob = DuctProblem(nx, ny, nz, 0.8, mask, n_steps=steps, window=(1, steps), checkpoint_every=2)
+    J, gi, gu = objective(prob, ui, u0, "f64", grad=True)
+    assert J == pytest.approx(Jt.item(), rel=1e-9)
+    for a, b in ((gi, tui.grad.numpy()), (gu, tu0.grad.numpy())):
+        assert np.linalg.norm(a - b) <= 1e-9 * np.linalg.norm(b)
+
+
 def test_adjoint_matches_central_differences(gpu):
     """A 64x32x32 copy of the adjoint case (sphere r=5 at (16,16,16)), 120 steps,
     drag averaged over steps 100-120: directional derivatives along random
