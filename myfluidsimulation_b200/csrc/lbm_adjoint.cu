@@ -122,7 +122,7 @@ __global__ void adj_init(AdjP<R> p, const double* __restrict__ u0, R* __restrict
 // outside the window, or recomputed) adds the block's drag sum (FP64).
 // Bound by HBM/L2: the state is read once and written once.
 template <class R, class IDX>
-__global__ void __launch_bounds__(256) adj_fwd(AdjP<R> p, const R* __restrict__ f, R* __restrict__ fn,
+__global__ void __launch_bounds__(256) adj_fwd(AdjP<R> p, const R* f, R* fn,
                                                const double* __restrict__ uin, double* __restrict__ drag_part) {
     step_begin();
     double drag = 0.0;
@@ -198,9 +198,8 @@ __global__ void __launch_bounds__(1024) adj_sum(const double* __restrict__ v, in
 // one reverse step, one cell per thread: lam0 = (d f'/d f)^T lam1 (+ the drag
 // term when wdrag != 0).  Bound by HBM/L2: f and lam1 read, lam0 written.
 template <class R, class IDX>
-__global__ void __launch_bounds__(256) adj_bwd(AdjP<R> p, const R* __restrict__ f, const R* __restrict__ lam1,
-                                               R* __restrict__ lam0, const double* __restrict__ uin,
-                                               double* __restrict__ g_uin, R wdrag) {
+__global__ void __launch_bounds__(256) adj_bwd(AdjP<R> p, const R* f, const R* lam1, R* lam0,
+                                               const double* __restrict__ uin, double* g_uin, R wdrag) {
     step_begin();
     const IDX N = (IDX)p.N;
     const int64_t id64 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;

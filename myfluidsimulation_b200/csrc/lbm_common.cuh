@@ -104,6 +104,10 @@ __device__ __forceinline__ uint32_t cvt_rs_bf16x2(float lo, float hi, uint32_t r
 // 5971 -> 5870 (HOME, inlet), 201x93x77 F16 956 -> 918, 64^3 159 -> 136 (Legacy) and
 // 186 -> 179 (HOME), 128x128x96 with the reference's table 556 -> 537.  The batched step,
 // one persistent launch, lost 1 % with it and is launched plainly.
+// What the steps write (populations, moments, adjoint fields) is read with coherent loads in
+// these kernels, never with __ldg or through a const __restrict__ pointer: that path wants
+// data that no one writes while the kernel runs, and it runs from before its wait on.  (__ldca
+// is scheduled as __ldg is; with plain loads the FP32 odd step with a mask takes 1.5 % longer.)
 __device__ __forceinline__ void step_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void step_next() { asm volatile("griddepcontrol.launch_dependents;"); }
 __device__ __forceinline__ void step_begin() {
@@ -153,7 +157,7 @@ __device__ __forceinline__ float feq_ref(int q, float rho, float ux, float uy, f
 struct StoreF32 {
     using T = float;
     static constexpr int kId = 0;
-    __device__ __forceinline__ static float ld(const T* p, int q, float r0) { return __ldg(p); }
+    __device__ __forceinline__ static float ld(const T* p, int q, float r0) { return __ldca(p); }
     // Every population store is streaming (.cs, evict first): nothing reads a
     // stored slot again in the same launch, and the step's state is larger than
     // L2, so the lines L2 keeps are those still to be gathered (the odd step's
@@ -181,7 +185,7 @@ struct StoreF32 {
 struct StoreF64 {
     using T = double;
     static constexpr int kId = 3;
-    __device__ __forceinline__ static double ld(const T* p, int q, float r0) { return __ldg(p); }
+    __device__ __forceinline__ static double ld(const T* p, int q, float r0) { return __ldca(p); }
     __device__ __forceinline__ static void st(T* p, int q, float r0, double v) { __stcs(p, v); }
     __device__ __forceinline__ static void ld2(const T* p, int q, float r0, double* o) {
         const double2 v = *reinterpret_cast<const double2*>(p);
@@ -291,7 +295,7 @@ template <class ST> struct Raw;
 template <> struct Raw<StoreF32> {   // FP32 stores f itself (S = 1, no shift)
     using T = float;
     static constexpr float S = 1.0f, invS = 1.0f;
-    __device__ __forceinline__ static float ld(const T* p) { return __ldg(p); }
+    __device__ __forceinline__ static float ld(const T* p) { return __ldca(p); }
     __device__ __forceinline__ static void st(T* p, float g) { __stcs(p, g); }
 };
 template <> struct Raw<StoreF16> {

@@ -199,9 +199,9 @@ template <> struct MomStore<__half> {
 };
 template <> struct MomStore<double> {
     static constexpr float S = 1.0f, invS = 1.0f;
-    __device__ __forceinline__ static double ld(const double* p) { return __ldg(p); }
+    __device__ __forceinline__ static double ld(const double* p) { return __ldca(p); }
     __device__ __forceinline__ static D2 ld2(const double* p) {
-        const double2 v = __ldg(reinterpret_cast<const double2*>(p));
+        const double2 v = __ldca(reinterpret_cast<const double2*>(p));
         return {v.x, v.y};
     }
 };
@@ -349,8 +349,8 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 8 ? 2 : 4) home_step(HomePara
     extern __shared__ __align__(16) unsigned char smraw[];
     step_wait();
     E* sm = reinterpret_cast<E*>(smraw);
-    const T* __restrict__ m = static_cast<const T*>(p.m);
-    T* __restrict__ mn = static_cast<T*>(p.mn);
+    const T* m = static_cast<const T*>(p.m);
+    T* mn = static_cast<T*>(p.mn);
     const IDX N = (IDX)p.N;
     const int nx = p.nx, ny = p.ny, nz = p.nz;
     const E omw = E(1) - E(p.omega);    // 1 - omega (in FP64 for the FP64 form)

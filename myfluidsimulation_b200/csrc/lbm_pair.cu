@@ -86,8 +86,7 @@ __device__ __forceinline__ float inlet_value(int q, float r, float kin) { return
 // VEC: nx is even, so a pair's two cells are one aligned 8-byte word of every plane.
 // MASK: the grid has solid cells, a band or a duct's ends (flags and links).
 template <bool MASK, bool VEC>
-__global__ void __launch_bounds__(NT, NB) aa_pair(AAParams p, const float* __restrict__ fa, float* __restrict__ fb,
-                                                  int zchunk) {
+__global__ void __launch_bounds__(NT, NB) aa_pair(AAParams p, const float* fa, float* fb, int zchunk) {
     extern __shared__ __align__(16) float sm[];
     step_begin();
     const int nx = p.nx, ny = p.ny, nz = p.nz;
@@ -164,26 +163,26 @@ __global__ void __launch_bounds__(NT, NB) aa_pair(AAParams p, const float* __res
                 const uint32_t s = place(qi), own = (uint32_t)q * N + zb[1];
                 const uint32_t s0 = s + (uint32_t)(cx(q) == 0 ? 0 : (cx(q) > 0 ? dm : d1));
                 const uint32_t s1 = s + (uint32_t)(cx(q) == 0 ? d1 : (cx(q) > 0 ? 0 : d2));
-                v[q].x = __ldg(at(fa, ((lk0 >> opp(q)) & 1u) ? own + cell0 : s0));
-                if (pair) v[q].y = __ldg(at(fa, ((lk1 >> opp(q)) & 1u) ? own + cell1 : s1));
+                v[q].x = __ldca(at(fa, ((lk0 >> opp(q)) & 1u) ? own + cell0 : s0));
+                if (pair) v[q].y = __ldca(at(fa, ((lk1 >> opp(q)) & 1u) ? own + cell1 : s1));
             });
         } else if (pair) {
             static_for<0, 19>([&](auto qi) {
                 constexpr int q = decltype(qi)::value;
                 const float* const s = from(qi);
                 if constexpr (cx(q) == 0) {
-                    if constexpr (VEC) v[q] = __ldg(reinterpret_cast<const float2*>(s));
-                    else v[q] = make_float2(__ldg(s), __ldg(s + d1));
+                    if constexpr (VEC) v[q] = __ldca(reinterpret_cast<const float2*>(s));
+                    else v[q] = make_float2(__ldca(s), __ldca(s + d1));
                 } else if constexpr (cx(q) > 0) {
-                    v[q] = make_float2(__ldg(s + dm), __ldg(s));
+                    v[q] = make_float2(__ldca(s + dm), __ldca(s));
                 } else {
-                    v[q] = make_float2(__ldg(s + (VEC ? 1 : d1)), __ldg(s + d2));
+                    v[q] = make_float2(__ldca(s + (VEC ? 1 : d1)), __ldca(s + d2));
                 }
             });
         } else {
             static_for<0, 19>([&](auto qi) {
                 constexpr int q = decltype(qi)::value;
-                v[q].x = __ldg(from(qi) + (cx(q) == 0 ? 0 : (cx(q) > 0 ? dm : d1)));
+                v[q].x = __ldca(from(qi) + (cx(q) == 0 ? 0 : (cx(q) > 0 ? dm : d1)));
             });
         }
     };
@@ -338,8 +337,8 @@ __global__ void __launch_bounds__(NT, NB) aa_pair(AAParams p, const float* __res
 }
 
 // the solid cells' populations into the second buffer (the two-step kernel does not touch them)
-__global__ void __launch_bounds__(256) pair_solids(const uint8_t* __restrict__ flags, const float* __restrict__ fa,
-                                                   float* __restrict__ fb, int64_t N) {
+__global__ void __launch_bounds__(256) pair_solids(const uint8_t* __restrict__ flags, const float* fa, float* fb,
+                                                   int64_t N) {
     step_begin();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= N || !(flags[i] & F_SOLID)) return;

@@ -41,7 +41,7 @@ __host__ __device__ constexpr uint32_t far_bit(int q) {
 // it.  (With the solid flags of the neighbours looked up per direction in 64-bit
 // arithmetic, and rows of 256 threads, 128 x 128 x 96 cells took 279 us.)
 template <int MODE, class IDX>
-__global__ void __launch_bounds__(256, 4) ref_push(AAParams p, const float* __restrict__ fa, float* __restrict__ fb) {
+__global__ void __launch_bounds__(256, 4) ref_push(AAParams p, const float* fa, float* fb) {
     constexpr bool MACRO = MODE >= 1, STATS = MODE == 2;
     step_begin();
     const IDX N = (IDX)p.N;
