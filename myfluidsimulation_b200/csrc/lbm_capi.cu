@@ -2,8 +2,8 @@
 //
 // One lbm_solver replaces the reference's three classes (src/lbm/lbm3d_legacy.hpp,
 // lbm3d_home.hpp, lbm3d_hybrid.hpp).  Memory per cell:
-//   Legacy/Hybrid: one population buffer (AA pattern; F32 with halfway bounce-back a
-//                  second one for two steps per pass), 19 x 4 B (F32) or 19 x 2 B
+//   Legacy/Hybrid: one population buffer (AA pattern; a second one in F32 with halfway
+//                  bounce-back while two steps per pass apply), 19 x 4 B (F32) or 19 x 2 B
 //                  (F16/BF16), plus rho,u,v,w (16 B), mask, flags (1 B each) and a
 //                  link word (4 B); the reference holds two population buffers.
 //   HOME:          two moment buffers of 10 x 4 B (or 10 x 2 B), as the reference.
@@ -42,7 +42,10 @@ struct lbm_solver {
     size_t esize = 4;
 
     void* f = nullptr;          // AA populations (reference bounce: buffer A)
-    void* f2 = nullptr;         // reference bounce: buffer B; F32 halfway: two-step passes (may be null)
+    void* f2 = nullptr;         // reference bounce: buffer B; F32 halfway: two-step passes (null where none are taken)
+    bool f2_used = false;       // a two-step pass has been queued or captured with f2
+    bool f2_failed = false;     // there was no memory for f2
+    bool in_batch = false;      // an instance of a batch, which steps in f alone
     void* m[2] = {nullptr, nullptr};   // HOME moments
     int cur = 0;
     float* macro = nullptr;     // 4*N floats: rho, ux, uy, uz (AA; HOME F16/BF16 export)
@@ -146,6 +149,51 @@ int home_after_step(lbm_solver* s) {
     return macro_fields(s, &b);
 }
 
+// whether calls of several steps take two-step passes
+bool pairs_apply(const lbm_solver* s) {
+    return is_aa(s) && !is_ref_push(s) && !s->zghost &&
+           lbm::pair_zchunk(s->dom.nx, s->dom.ny, s->dom.nz, s->storage, s->use_flags) > 0;
+}
+
+// The second buffer of the two-step passes, taken if it is not there; without
+// memory for it every step is a single one.  Allowed while a stream captures:
+// nothing is queued here.
+int take_pair_buffer(lbm_solver* s) {
+    if (s->f2 || s->f2_failed) return LBM_OK;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    CK(cudaThreadExchangeStreamCaptureMode(&mode));
+    const bool ok = cudaMalloc(&s->f2, s->esize * 19 * (size_t)s->N) == cudaSuccess;
+    const cudaError_t e = ok ? lbm::pair_prepare() : cudaSuccess;
+    CK(cudaThreadExchangeStreamCaptureMode(&mode));
+    if (!ok) {
+        cudaGetLastError();
+        s->f2 = nullptr;
+        s->f2_failed = true;
+    }
+    CK(e);
+    return LBM_OK;
+}
+
+// Holds that buffer while its passes apply: taken when a mask, a band or ghost
+// planes let them, given back when they no longer do, unless work with its
+// address is queued or captured.  A solver in a batch takes it only for a call
+// of its own (enqueue_steps).
+int fit_pair_buffer(lbm_solver* s) {
+    if (!is_aa(s) || is_ref_push(s)) return LBM_OK;
+    s->f2_failed = false;
+    if (pairs_apply(s) && !s->in_batch) return take_pair_buffer(s);
+    if (s->f2 && !s->f2_used) {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusActive;
+        if (cudaStreamIsCapturing(s->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+            cudaGetLastError();      // (no memory can be given back now)
+            return LBM_OK;
+        }
+        CK(cudaFree(s->f2));
+        s->f2 = nullptr;
+    }
+    return LBM_OK;
+}
+
 int rebuild_flags(lbm_solver* s) {
     s->use_flags = s->any_solid || s->bc == LBM_BC_DUCT || (s->method == LBM_METHOD_HYBRID && s->any_band);
     if (!s->home_zchunk_set) s->home_zchunk = s->home_auto[s->use_flags];
@@ -153,7 +201,7 @@ int rebuild_flags(lbm_solver* s) {
                                (s->method == LBM_METHOD_HYBRID && s->any_band) ? s->band : nullptr, s->flags,
                                s->links, s->dom.nx, s->dom.ny, s->dom.nz, s->bc == LBM_BC_DUCT, s->stream));
     drop_graph(s);
-    return LBM_OK;
+    return fit_pair_buffer(s);
 }
 
 lbm::AAParams aa_params(lbm_solver* s, bool macro, bool stats) {
@@ -231,8 +279,14 @@ static int enqueue_pairs(lbm_solver* s, bool first) {
 }
 
 static int enqueue_steps(lbm_solver* s, int n) {
-    const bool pairs = is_aa(s) && !is_ref_push(s) && s->f2 && !s->zghost &&
-                       lbm::pair_zchunk(s->dom.nx, s->dom.ny, s->dom.nz, s->storage, s->use_flags) > 0;
+    // (one step at an even parity comes first)
+    bool pairs = n - (s->parity == 0 ? 1 : 0) - (s->macro_out || s->stats_on ? 1 : 0) >= 4 && pairs_apply(s);
+    if (pairs) {
+        const int rc = take_pair_buffer(s);
+        if (rc != LBM_OK) return rc;
+        pairs = s->f2 != nullptr;
+        if (pairs) s->f2_used = true;
+    }
     bool first_pair = true;
     for (int i = 0; i < n; ++i) {
         // steps behind an odd parity and before one that writes macro fields or statistics
@@ -436,16 +490,6 @@ int lbm_create(const lbm_domain* dom, const lbm_options* opts, lbm_solver** out)
         (is_ref_push(s) && cudaMemsetAsync(s->f2, 0, s->esize * 19 * (size_t)N, s->stream) != cudaSuccess)) {
         set_error("lbm_create: cudaMemset failed");
         return fail(LBM_ERR_CUDA);
-    }
-    // the second buffer of the two-step kernel; without it every step is a single one
-    if (is_aa(s) && !is_ref_push(s) && lbm::pair_zchunk(dom->nx, dom->ny, dom->nz, o.storage, false) > 0) {
-        if (!dmalloc(&s->f2, s->esize * 19 * (size_t)N)) {
-            cudaGetLastError();
-            s->f2 = nullptr;
-        } else if (lbm::pair_prepare() != cudaSuccess) {
-            set_error("lbm_create: cannot set the two-step kernel's shared-memory size");
-            return fail(LBM_ERR_CUDA);
-        }
     }
     if (!is_aa(s) && lbm::home_prepare() != cudaSuccess) {
         set_error("lbm_create: cannot set the HOME kernel's shared-memory size");
@@ -793,7 +837,7 @@ int lbm_set_z_ghosts(lbm_solver* s, int on) {
     if (on && s->dom.nz < 3) { set_error("lbm_set_z_ghosts: needs nz >= 3 (two ghost planes)"); return LBM_ERR_INVALID; }
     s->zghost = on != 0;
     drop_graph(s);
-    return LBM_OK;
+    return fit_pair_buffer(s);
 }
 
 int lbm_zslab_slots(lbm_solver* s, int plane, int cz, void** ptrs, int64_t* bytes) {
@@ -1314,8 +1358,12 @@ int lbm_batch_create(lbm_solver* const* solvers, int32_t n, void* stream, lbm_ba
         b->own_stream = true;
     }
     // the instances' own streams finish their queued work first
-    for (lbm_solver* s : b->inst)
+    for (lbm_solver* s : b->inst) {
         if (cudaStreamSynchronize(s->stream) != cudaSuccess) { lbm_batch_destroy(b); set_error("lbm_batch_create: sync"); return LBM_ERR_CUDA; }
+        s->in_batch = true;
+        const int rc = fit_pair_buffer(s);
+        if (rc != LBM_OK) { lbm_batch_destroy(b); return rc; }
+    }
     if (cudaMalloc((void**)&b->d_params, sizeof(lbm::AAParams) * n) != cudaSuccess ||
         cudaMalloc((void**)&b->d_stats, sizeof(double) * lbm::NSTAT * n) != cudaSuccess) {
         lbm_batch_destroy(b);

@@ -1,0 +1,89 @@
+"""The second population buffer of the two-step passes (76 bytes a cell, FP32): held by the
+solvers whose calls take such passes, and by no others -- z-slabs, instances of a batch, ducts
+and masked grids that stay in L2."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from myfluidsimulation_b200 import lib
+from myfluidsimulation_b200.solvers import BC_DUCT, METHOD_HYBRID, METHOD_LEGACY, Batch, Solver
+
+pytestmark = pytest.mark.gpu
+
+DIMS = (128, 128, 96)
+N = int(np.prod(DIMS))
+
+
+def held(make, keep):
+    """Bytes of device memory a cell that make() takes."""
+    import torch
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    keep.append(make())
+    torch.cuda.synchronize()
+    return (before - torch.cuda.mem_get_info()[0]) / N
+
+
+def wall():
+    m = np.zeros(DIMS[::-1], np.uint8)
+    m[:, 0, :] = 9
+    return m
+
+
+def slab():
+    s = Solver(*DIMS, 0.6)
+    assert lib().lbm_set_z_ghosts(s._h, 1) == 0
+    return s
+
+
+def masked():
+    s = Solver(*DIMS, 0.6)
+    s.set_solid_mask(wall())
+    return s
+
+
+@pytest.mark.parametrize("make,pairs", [
+    (lambda: Solver(*DIMS, 0.6), True),
+    (lambda: Solver(*DIMS, 0.6, method=METHOD_HYBRID), True),
+    (lambda: Solver(*DIMS, 0.6, bc=BC_DUCT, inlet_u=0.04), False),
+    (slab, False),
+    (masked, False),
+])
+def test_memory_is_held_where_two_step_passes_apply(gpu, make, pairs):
+    import torch
+    torch.cuda.mem_get_info()
+    make().close()      # (what the first solver of a process loads)
+    keep = []
+    b = held(make, keep)      # 99 bytes a cell without the buffer, 175 with it
+    assert 165 < b < 195 if pairs else 90 < b < 120
+    s = keep[0]
+    if make is slab:      # switched back, the passes apply again
+        assert held(lambda: lib().lbm_set_z_ghosts(s._h, 0), []) > 66
+    if make is masked:
+        assert held(lambda: s.set_solid_mask(np.zeros_like(wall())), []) > 66
+    s.close()
+
+
+def test_batched_instances_hold_none_and_still_step_alone(gpu):
+    rng = np.random.default_rng(4)
+    f = [(1 + 1e-3 * rng.standard_normal(DIMS[::-1])).astype(np.float32)]
+    f += [(1e-2 * rng.standard_normal(DIMS[::-1])).astype(np.float32) for _ in range(3)]
+    Solver(*DIMS, 0.6).close()
+    keep = []
+    assert held(lambda: [Solver(*DIMS, 0.6) for _ in range(2)], keep) > 2 * 165
+    a, b = keep[0]
+    assert held(lambda: Batch([a, b]), keep) < -2 * 66
+    a.reinit_from_host(*f)
+    b.reinit_from_host(*f)
+    keep[1].refresh()
+    keep[1].step(8)
+    keep[1].synchronize()
+    one = Solver(*DIMS, 0.6)
+    one.reinit_from_host(*f)
+    one.step(8)
+    for s in (a, one):      # an instance's own call takes the buffer again
+        s.step(9)
+    np.testing.assert_array_equal(a.state(), one.state())
+    for s in (keep[1], a, b, one):
+        s.close()
