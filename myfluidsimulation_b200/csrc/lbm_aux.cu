@@ -2,6 +2,8 @@
 // flag/link words built from the solid mask, the B0 band, the final pass of
 // the FP64 statistics, and the reference's free device helpers
 // (reinit_equilibrium_from_macro, launch_speed, make_rho_gauss/slab).
+#include <cuda.h>
+
 #include <mutex>
 
 #include "lbm_common.cuh"
@@ -20,28 +22,51 @@ int num_sms() {
     return n;
 }
 
+namespace {
+// Identity of the current context, never given again to another one.
+bool context_id(unsigned long long* id) {
+    static const auto get = [] {
+        void* fn = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &fn, 12000, cudaEnableDefault, &found) != cudaSuccess) fn = nullptr;
+        return reinterpret_cast<decltype(&cuCtxGetId)>(fn);
+    }();
+    return get && get(nullptr, id) == CUDA_SUCCESS;
+}
+}  // namespace
+
 cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s) {
-    constexpr int kDevices = 64;
+    // One pool per context: cudaDeviceReset ends a context and its pools with it, and what
+    // comes after it on the same device is another one.
+    struct Kept {
+        unsigned long long context;
+        cudaMemPool_t pool;
+    };
+    constexpr int kContexts = 64;
     static std::mutex mu;
-    static cudaMemPool_t pools[kDevices] = {};
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    if (dev >= kDevices) return cudaMallocAsync(p, bytes, s);
+    static Kept kept[kContexts];
+    static int n = 0;
+    unsigned long long id = 0;
+    if (!context_id(&id)) return cudaMallocAsync(p, bytes, s);
     cudaMemPool_t pool = nullptr;
     {
         std::lock_guard<std::mutex> g(mu);
-        if (!pools[dev]) {
+        for (int i = 0; i < n; ++i)
+            if (kept[i].context == id) pool = kept[i].pool;
+        if (!pool) {
+            if (n == kContexts) return cudaMallocAsync(p, bytes, s);
+            int dev = 0;
+            cudaError_t e = cudaGetDevice(&dev);
             cudaMemPoolProps props{};
             props.allocType = cudaMemAllocationTypePinned;
             props.location.type = cudaMemLocationTypeDevice;
             props.location.id = dev;
-            e = cudaMemPoolCreate(&pools[dev], &props);
-            if (e != cudaSuccess) { pools[dev] = nullptr; return e; }
+            if (e == cudaSuccess) e = cudaMemPoolCreate(&pool, &props);
+            if (e != cudaSuccess) return e;
             uint64_t keep = kScratchKept;
-            cudaMemPoolSetAttribute(pools[dev], cudaMemPoolAttrReleaseThreshold, &keep);
+            cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+            kept[n++] = {id, pool};
         }
-        pool = pools[dev];
     }
     return cudaMallocFromPoolAsync(p, bytes, pool, s);
 }

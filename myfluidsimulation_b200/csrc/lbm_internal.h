@@ -139,7 +139,7 @@ cudaError_t launch_voxelize(const float* d_tris, int64_t ntri, const float* bb, 
 int num_sms();
 
 // Scratch memory of one call, from the library's own stream-ordered pool of the
-// current device (free it with cudaFreeAsync).  Up to kScratchKept bytes stay with
+// current context (free it with cudaFreeAsync).  Up to kScratchKept bytes stay with
 // the pool across calls, the rest goes back at the next synchronisation: the
 // default pool gives everything back each time, which made a call that allocates,
 // runs 0.45 ms of kernels and waits take 1.3-2.9 ms.  Safe from any thread and stream.
