@@ -107,10 +107,13 @@ def duct_sphere_mesh(nx: int, ny: int, nz: int, radius: float, center, levels: i
 
 def duct_mask(nx: int, ny: int, nz: int, obstacle: np.ndarray | None = None) -> np.ndarray:
     """Mask (nz, ny, nx) uint8: walls on the y and z faces (1|8), obstacle cells 1."""
-    if obstacle is None:
+    hit = None if obstacle is None else obstacle.reshape(nz, ny, nx) != 0
+    if type(hit) is np.ndarray and hit.dtype == bool:      # MASK_SOLID is 1: the comparison's own bytes
+        m = np.ascontiguousarray(hit).view(np.uint8)
+    else:      # none, or a form with a comparison of its own (torch tensors, masked arrays)
         m = np.zeros((nz, ny, nx), dtype=np.uint8)
-    else:      # MASK_SOLID (1) where the obstacle is not 0: the comparison's own bytes
-        m = np.not_equal(obstacle.reshape(nz, ny, nx), 0, order="C").view(np.uint8)
+        if hit is not None:
+            m[hit] = MASK_SOLID
     wall = MASK_SOLID | MASK_WALL
     m[:, 0, :] = wall
     m[:, ny - 1, :] = wall
