@@ -76,6 +76,7 @@ def _run(problem: DuctProblem, precision, ui, u0, gi, gu) -> float:
 
 def _autograd_function():
     import torch
+    direct = (torch.float16, torch.float32, torch.float64)      # other types: as numpy takes (or refuses) them
 
     class DragObjective(torch.autograd.Function):
         """J(u_inlet, u0) with the library's adjoint as its backward."""
@@ -83,10 +84,10 @@ def _autograd_function():
         @staticmethod
         def forward(ctx, u_inlet, u0, problem, precision="f32"):
             here = torch.cuda.current_device() if u_inlet.is_cuda and u0.is_cuda else None
-            if here is not None and u_inlet.device.index == here and u0.device.index == here:
+            if here is not None and all(t.device.index == here and t.dtype in direct for t in (u_inlet, u0)):
                 # the controls are where the library runs: no copies through the host
                 nx, ny, nz = problem.nx, problem.ny, problem.nz
-                ui, u = [t.detach().to(torch.float64).contiguous() for t in (u_inlet, u0)]
+                ui, u = [t.detach().to(torch.float64).resolve_neg().contiguous() for t in (u_inlet, u0)]
                 if ui.numel() != ny * nz or u.numel() != 3 * nx * ny * nz:
                     raise ValueError("mask, u_inlet or u0 has the wrong size")
                 gi = torch.empty((nz, ny), dtype=torch.float64, device=u.device)

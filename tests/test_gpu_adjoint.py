@@ -122,6 +122,23 @@ def test_device_controls_equal_host_controls(gpu, tiny, dtype):
         drag_objective(torch.zeros(3, 3, device="cuda"), torch.zeros(3, device="cuda"), prob)
 
 
+def test_device_controls_of_other_forms(gpu, tiny):
+    """Controls on the GPU whose memory does not hold their values (a negative view) count by value; types that
+    numpy has no counterpart of are refused there as they are on the CPU."""
+    import torch
+    prob, ui, u0 = tiny
+    a, b = torch.tensor(ui, device="cuda"), torch.tensor(u0, device="cuda")
+    want = drag_objective(a, b, prob, "f64")
+    neg = torch._neg_view((-a).contiguous())
+    assert neg.is_neg()
+    assert drag_objective(neg, b, prob, "f64").item() == want.item()
+    assert drag_objective(a, torch._neg_view(-b), prob, "f64").item() == want.item()
+    for dev in ("cpu", "cuda"):
+        with pytest.raises(TypeError):
+            drag_objective(a.to(dev, torch.bfloat16), b.to(dev, torch.bfloat16), prob)
+    assert drag_objective(a.half(), b.half(), prob, "f64").item() == drag_objective(a.half().cpu(), b.half().cpu(), prob, "f64").item()
+
+
 @pytest.mark.parametrize("seed", [1, 2])
 def test_fp32_gradient_carries_no_bias_of_the_weights(gpu, seed):
     """The FP32 weights add up to 1 + 1.5e-8 (their own rounding): taken as they are, each reverse step adds a relative
