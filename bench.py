@@ -59,14 +59,26 @@ RADIUS, CENTER = 16, (64, 64, 64)
 B0 = 2
 # algorithmic bytes per cell of one pass (state read once + written once, plus the mask/flag byte)
 BYTES = {"legacy": 19 * 4 * 2 + 1, "hybrid": 19 * 4 * 2 + 1, "home": 10 * 4 * 2 + 1}
-KERNEL = {"legacy": "aa_pair", "hybrid": "aa_pair", "home": "home_step"}
-# LBM step kernels of one 50-step interval.  On the duct Legacy/Hybrid take the first step and the
-# one with the statistics singly, and the 48 between them two at a time (aa_pair), each pass one read and one
-# write of the state; HOME takes every step singly.
-PASSES = {"legacy": {"aa_even": 1, "aa_pair": 24, "aa_odd": 1}, "home": {"home_step": DRAG_EVERY}}
-PASSES["hybrid"] = PASSES["legacy"]
-# plus the statistics' final pass and, for Legacy/Hybrid, pair_solids (copies what solid cells hold) once
-LAUNCHES = {"legacy": 26 + 2, "hybrid": 26 + 2, "home": DRAG_EVERY + 1}
+# LBM step kernels of one 50-step interval that starts at an even parity and makes `passes` passes over
+# the state: a pass of aa_pair takes two steps, the others one each (aa_even and aa_odd alternate).  On
+# the duct Legacy/Hybrid take the first step and the one with the statistics singly and the 48 between them two at a time.
+def kernels_of(method, passes):
+    if method == "home":
+        return {"home_step": passes}
+    pairs = DRAG_EVERY - passes
+    singles = passes - pairs
+    return {"aa_even": (singles + 1) // 2, "aa_pair": pairs, "aa_odd": singles // 2}
+
+
+# all launches of that interval: plus the statistics' final pass and, with aa_pair, pair_solids (copies what solid cells hold)
+def launches_of(method, passes):
+    return passes + 1 + (1 if passes < DRAG_EVERY else 0)
+
+
+def main_kernel(method, passes):
+    return "home_step" if method == "home" else ("aa_pair" if passes < DRAG_EVERY else "aa_even/aa_odd")
+
+
 METRIC = "D3Q19 MLUPS (Legacy BGK FP32, duct 256x128x128 past a voxelized sphere)"
 WORKLOAD_TEXT = {
     "periodic": "duct 256x128x128, y/z walls as solid cells, icosphere (5120 triangles, r=16, centre (64,64,64)) "
@@ -204,9 +216,9 @@ def kernel_split(s, method, torch, launches=40):
 
     HOME: one lbm_step(launches) call between two CUDA events.  AA methods: the
     same over single-step calls, split into even and odd by a second pass with a
-    CUDA event between every two (no synchronisation inside the loop); then one
-    call of 2 x launches steps from an odd parity, which is `launches` passes of
-    aa_pair (and one pair_solids).  No macro fields, no statistics.  Returns
+    CUDA event between every two (no synchronisation inside the loop); then,
+    where two steps per pass apply, one call of 2 x launches steps from an odd
+    parity, which is `launches` passes of aa_pair (and one pair_solids).  No macro fields, no statistics.  Returns
     {kernel: us per launch}."""
     st = torch.cuda.current_stream()
     s.enable_stats(False)
@@ -235,20 +247,21 @@ def kernel_split(s, method, torch, launches=40):
         ev[i + 1].record(st)
     torch.cuda.synchronize()
     t = [1e3 * ev[i].elapsed_time(ev[i + 1]) for i in range(launches)]
+    a, b = statistics.median(t[0::2]), statistics.median(t[1::2])
+    names = ("aa_even", "aa_odd") if par == 0 else ("aa_odd", "aa_even")
+    split = {names[0]: round(2 * mean_us * a / (a + b), 2), names[1]: round(2 * mean_us * b / (a + b), 2)}
     if s.steps % 2 == 0:
         s.step(1)
-    e0.record(st)
-    s.step(2 * launches)               # a multiple of four
-    e1.record(st)
-    torch.cuda.synchronize()
-    pair_us = 1e3 * e0.elapsed_time(e1) / launches
+    if s.step_passes(2 * launches) == launches:      # (a multiple of four steps, all of them in pairs)
+        e0.record(st)
+        s.step(2 * launches)
+        e1.record(st)
+        torch.cuda.synchronize()
+        split["aa_pair"] = round(1e3 * e0.elapsed_time(e1) / launches, 2)
     s.step(1)                          # back to an even parity
     s.set_macro_output(True)
     s.enable_stats(True)
-    a, b = statistics.median(t[0::2]), statistics.median(t[1::2])
-    names = ("aa_even", "aa_odd") if par == 0 else ("aa_odd", "aa_even")
-    return {names[0]: round(2 * mean_us * a / (a + b), 2), names[1]: round(2 * mean_us * b / (a + b), 2),
-            "aa_pair": round(pair_us, 2)}
+    return split
 
 
 def run_method(method, workload, mask, args, torch, dist=None):
@@ -256,6 +269,7 @@ def run_method(method, workload, mask, args, torch, dist=None):
     s, nb = make_solver(method, workload, mask, st.cuda_stream)
     for _ in range(args.warmup):
         s.step(DRAG_EVERY)
+    passes = s.step_passes(DRAG_EVERY)
     torch.cuda.synchronize()
     if dist:
         dist.barrier()
@@ -271,7 +285,7 @@ def run_method(method, workload, mask, args, torch, dist=None):
         dist.barrier()
     ms = e0.elapsed_time(e1)
     st_ = s.stats()
-    res = {"ms_total": ms, "launches": args.steps * LAUNCHES[method], "band_cells": nb,
+    res = {"ms_total": ms, "launches": args.steps * launches_of(method, passes), "passes": passes, "band_cells": nb,
            "drag_last": [st_["drag_x"], st_["drag_y"], st_["drag_z"]], "mass": st_["mass"],
            "kernel_us": kernel_split(s, method, torch)}
     return s, res
@@ -1230,19 +1244,19 @@ def main():
         ms = float(ms.item())
         cell_updates = N * DRAG_EVERY * args.steps * world
         mlups = cell_updates / (ms * 1e-3) / 1e6
-        passes = sum(PASSES[mth].values())
+        passes = r["passes"]
         per_pass_ms = r["ms_total"] / (passes * args.steps)
         achieved = N * BYTES[mth] / (per_pass_ms * 1e-3) / 1e9
         tr = profile_traffic(mth)
         ku = r["kernel_us"]
-        split_ms = sum(n * ku[k] for k, n in PASSES[mth].items()) / 1e3
+        split_ms = sum(n * ku[k] for k, n in kernels_of(mth, passes).items() if n) / 1e3
         results[key] = {"mlups": round(mlups, 1), "ms_per_step": round(ms / args.steps, 4),
                         "workload": wl, "kernel_us": ku,
                         "kernel_split_ms_per_step": round(split_ms, 4),
                         "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                                      "frac": round(achieved / peak, 4),
                                      "traffic": None if tr is None else int(round(tr * N)),
-                                     "kernel": KERNEL[mth], "bytes_per_cell": BYTES[mth],
+                                     "kernel": main_kernel(mth, passes), "bytes_per_cell": BYTES[mth],
                                      "passes_per_50_steps": passes},
                         "kernel_frac": {k: round(N * BYTES[mth] / (v * 1e-6) / 1e9 / peak, 4) for k, v in ku.items()},
                         "drag": [round(x, 6) for x in r["drag_last"]], "mass": round(r["mass"], 3),

@@ -194,6 +194,10 @@ int lbm_get_state(lbm_solver* s, float* host_out);
 int lbm_dims(lbm_solver* s, int32_t* nx, int32_t* ny, int32_t* nz, int64_t* n);
 /* Steps taken since the last reset/reinit. */
 int lbm_step_count(lbm_solver* s, int64_t* steps);
+/* Passes over the state that the next lbm_step(s, substeps) makes: one per step, or
+ * fewer where FP32 Legacy/Hybrid takes two steps per pass (and has the memory for it).
+ * No reference counterpart. */
+int lbm_step_passes(lbm_solver* s, int substeps, int* passes);
 
 /* Enables (1) or disables (0) the FP64 statistics of the last substep of
  * every lbm_step (mass, kinetic energy, momentum, momentum-exchange drag). */

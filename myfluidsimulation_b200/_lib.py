@@ -94,6 +94,7 @@ _PROTOS = [
     ("lbm_dims", C.c_int, [_P, C.POINTER(C.c_int32), C.POINTER(C.c_int32), C.POINTER(C.c_int32),
                            C.POINTER(C.c_int64)]),
     ("lbm_step_count", C.c_int, [_P, C.POINTER(C.c_int64)]),
+    ("lbm_step_passes", C.c_int, [_P, C.c_int, C.POINTER(C.c_int)]),
     ("lbm_enable_stats", C.c_int, [_P, C.c_int]),
     ("lbm_get_stats", C.c_int, [_P, _P]),
     ("lbm_get_stats_async", C.c_int, [_P, _P]),

@@ -155,6 +155,14 @@ bool pairs_apply(const lbm_solver* s) {
            lbm::pair_zchunk(s->dom.nx, s->dom.ny, s->dom.nz, s->storage, s->use_flags) > 0;
 }
 
+// How many groups of four steps a call of n takes in two passes each: those behind an
+// odd parity (one step at an even one comes first) and before a last step that writes
+// macro fields or statistics.
+int fours_in_pairs(const lbm_solver* s, int n) {
+    const int m = n - (s->parity == 0 ? 1 : 0) - (s->macro_out || s->stats_on ? 1 : 0);
+    return m >= 4 && !s->f2_failed && pairs_apply(s) ? m / 4 : 0;
+}
+
 // The second buffer of the two-step passes, taken if it is not there; without
 // memory for it every step is a single one.  Allowed while a stream captures:
 // nothing is queued here.
@@ -279,19 +287,16 @@ static int enqueue_pairs(lbm_solver* s, bool first) {
 }
 
 static int enqueue_steps(lbm_solver* s, int n) {
-    // (one step at an even parity comes first)
-    bool pairs = n - (s->parity == 0 ? 1 : 0) - (s->macro_out || s->stats_on ? 1 : 0) >= 4 && pairs_apply(s);
-    if (pairs) {
+    int fours = fours_in_pairs(s, n);
+    if (fours > 0) {
         const int rc = take_pair_buffer(s);
         if (rc != LBM_OK) return rc;
-        pairs = s->f2 != nullptr;
-        if (pairs) s->f2_used = true;
+        if (s->f2) s->f2_used = true;
+        else fours = 0;
     }
     bool first_pair = true;
     for (int i = 0; i < n; ++i) {
-        // steps behind an odd parity and before one that writes macro fields or statistics
-        while (pairs && s->parity == 1 &&
-               n - i - (s->macro_out || s->stats_on ? 1 : 0) >= 4) {
+        for (; fours > 0 && s->parity == 1; --fours) {
             const int rc = enqueue_pairs(s, first_pair);
             first_pair = false;
             if (rc != LBM_OK) return rc;
@@ -1126,6 +1131,12 @@ int lbm_dims(lbm_solver* s, int32_t* nx, int32_t* ny, int32_t* nz, int64_t* n) {
 int lbm_step_count(lbm_solver* s, int64_t* steps) {
     if (!s || !steps) { set_error("lbm_step_count: null argument"); return LBM_ERR_INVALID; }
     *steps = s->steps;
+    return LBM_OK;
+}
+
+int lbm_step_passes(lbm_solver* s, int substeps, int* passes) {
+    if (!s || !passes || substeps < 0) { set_error("lbm_step_passes: bad argument"); return LBM_ERR_INVALID; }
+    *passes = substeps - 2 * fours_in_pairs(s, substeps);
     return LBM_OK;
 }
 

@@ -158,6 +158,12 @@ class Solver:
         check(lib().lbm_step_count(self._h, C.byref(v)))
         return v.value
 
+    def step_passes(self, n: int) -> int:
+        """Passes over the state that the next step(n) makes (lbm_step_passes)."""
+        v = C.c_int()
+        check(lib().lbm_step_passes(self._h, int(n), C.byref(v)))
+        return v.value
+
     # -- outputs -----------------------------------------------------------------
     @property
     def stream(self) -> int:

@@ -87,3 +87,28 @@ def test_batched_instances_hold_none_and_still_step_alone(gpu):
     np.testing.assert_array_equal(a.state(), one.state())
     for s in (keep[1], a, b, one):
         s.close()
+
+
+def launches(s, n):
+    """Kernels that step(n) launches: the nodes of the graph it is captured into (not run)."""
+    rt = C.CDLL("libcudart.so.12")      # the one the library is linked to
+    st, graph, count = C.c_void_p(s.stream), C.c_void_p(), C.c_size_t()
+    assert rt.cudaStreamBeginCapture(st, 2) == 0      # relaxed
+    s.step(n)
+    assert rt.cudaStreamEndCapture(st, C.byref(graph)) == 0
+    assert rt.cudaGraphGetNodes(graph, None, C.byref(count)) == 0
+    assert rt.cudaGraphDestroy(graph) == 0
+    return count.value
+
+
+@pytest.mark.parametrize("make,pairs", [(lambda: Solver(*DIMS, 0.6), True), (masked, False), (slab, False)])
+def test_passes_are_reported_as_they_are_taken(gpu, make, pairs):
+    s = make()
+    for macros, calls in ((True, (1, 5, 6, 9, 10, 3)), (False, (5, 4, 4, 7, 1, 4, 3))):
+        s.set_macro_output(macros)
+        for n in calls:
+            told = s.step_passes(n)
+            assert launches(s, n) == told
+            assert told == n if not pairs or n < 4 else told <= n
+        assert s.step_passes(50) == (26 if pairs else 50)      # (an even parity, with macro fields 1 + 24 + 1)
+    s.close()
