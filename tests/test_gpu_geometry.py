@@ -99,3 +99,14 @@ def test_voxelizer_flood_fill_of_shells_vs_oracle(gpu, oracle, dims, refine):
     got = G.voxelize_mesh_to_mask(mesh, p)
     want = oracle.voxelize(shell, mesh_bbox(shell), dims, 0.9, (0.5, 0.5, 0.5), refine, 0.5)
     np.testing.assert_array_equal(got, want)
+
+
+@pytest.mark.parametrize("dims", [(40, 33, 1), (33, 1, 40), (1, 40, 33), (1, 1, 50), (40, 1, 1), (1100, 900, 1), (1100, 1, 900)])
+def test_voxelizer_grids_of_one_plane_vs_oracle(gpu, oracle, dims):
+    """One plane (or line) of cells, in shared and in global memory, through a ring with a gap and a closed one."""
+    tris = W.icosphere(2)
+    ring = tris[np.abs(tris.mean(1) - np.array([0.0, 0.0, 1.0])).max(1) > 0.5]
+    shell = np.concatenate([ring, tris * 0.6, tris[np.abs(tris.mean(1)[:, 0] - 1.0) > 0.5] * 0.8]).astype(np.float32)
+    mesh = G.mesh_from_triangles(shell)
+    got = G.voxelize_mesh_to_mask(mesh, G.VoxelParams(*dims, 0.9, (0.5, 0.5, 0.5), 1, 0.5))
+    np.testing.assert_array_equal(got, oracle.voxelize(shell, mesh_bbox(shell), dims, 0.9, (0.5, 0.5, 0.5), 1, 0.5))
