@@ -772,7 +772,7 @@ def vtk_study(args, torch):
     st = torch.cuda.current_stream()
     with tempfile.TemporaryDirectory() as td:
         mask, _, _ = build_mask(td)
-    s, _ = make_solver("legacy", "periodic", mask, st.cuda_stream)
+    s, _ = make_solver("legacy", "inlet", mask, st.cuda_stream)
     s.step(50)
     torch.cuda.synchronize()
     N = NX * NY * NZ
@@ -903,7 +903,7 @@ def render_study(args, torch):
     st = torch.cuda.current_stream()
     with tempfile.TemporaryDirectory() as td:
         mask, _, _ = build_mask(td)
-    s, _ = make_solver("legacy", "periodic", mask, st.cuda_stream)
+    s, _ = make_solver("legacy", "inlet", mask, st.cuda_stream)
     s.step(200)
     r, u, v, w = s.macro_ptrs()
     N = NX * NY * NZ
