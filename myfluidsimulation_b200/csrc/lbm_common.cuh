@@ -102,8 +102,9 @@ __device__ __forceinline__ uint32_t cvt_rs_bf16x2(float lo, float hi, uint32_t r
 // the next step's blocks are already there (180x434x244 3.49 against 3.33 ms per 7 steps).
 // Measured, us per 50, 20 or 10 steps: the 256x128x128 duct 5716 -> 5634 (Legacy) and
 // 5971 -> 5870 (HOME, inlet), 201x93x77 F16 956 -> 918, 64^3 159 -> 136 (Legacy) and
-// 186 -> 179 (HOME), 128x128x96 with the reference's table 556 -> 537.  The batched step,
-// one persistent launch, lost 1 % with it and is launched plainly.
+// 186 -> 179 (HOME), 128x128x96 with the reference's table 556 -> 537.  Steps replayed as a
+// graph gain nothing (64^3 HOME 105 us per 20 with it and without).  The batched step, one
+// persistent launch, lost 1 % with it and is launched plainly.
 // What the steps write (populations, moments, adjoint fields) is read with coherent loads in
 // these kernels, never with __ldg or through a const __restrict__ pointer: that path wants
 // data that no one writes while the kernel runs, and it runs from before its wait on.  (__ldca

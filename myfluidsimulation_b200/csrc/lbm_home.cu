@@ -717,9 +717,10 @@ int home_num_blocks(int nx, int ny, int nz, int zchunk) {
 // a (waves + 1/4)(zchunk + 2) + b blocks (zchunk + 2), the measured time of a step in us
 // to about 8 % (96^3 22.2 -> 20.4 us with 6 planes for 4, 128x128x96 42.4 -> 37.6, 201x93x77
 // 52.0 -> 49.1); longer ones leave too little to even out the blocks.  A grid whose blocks fill half the slots or less takes
-// that chunk even if it is shorter (32^3 7.3 -> 3.9); above that a shorter one costs other
-// solvers on the device what it gains alone (three 64^3 solvers side by side: 5.2 us a step
-// each with 4 planes, 7.1 with 3).  Blocks at walls and duct ends take longer, and longer
+// that chunk even if it is shorter (32^3 7.3 -> 3.9).  Above that 4 planes it is: a solver
+// alone loses up to 18 % by it where they leave 160 to 240 blocks (64x64x48 8.5 us, 7.1 with 3
+// planes, 7.5 with 2) and nothing at 256 (64^3 8.5, 9.2 with 3), but solvers side by side lose
+// more by the shorter one (three 64^3: 5.2 us a step each with 4 planes, 7.1 with 3).  Blocks at walls and duct ends take longer, and longer
 // chunks leave a long last wave (256x128x128 duct: 8 planes 116, 12 planes 113, 16 planes 130).
 int home_pick_zchunk(int nx, int ny, int nz, int blocks_per_sm, bool flags) {
     const int64_t slots = (int64_t)num_sms() * blocks_per_sm;

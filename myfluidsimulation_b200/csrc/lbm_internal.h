@@ -78,9 +78,6 @@ int64_t aa_odd_grid(int nx, int ny, int64_t planes, bool mask, int storage, Laun
 // without a mask, on the whole grid or as a z-slab of nz - 2 planes of its own.  (Fewer planes
 // can give more blocks: a shorter run of planes per block is chosen for them.)
 int64_t aa_stat_blocks(int nx, int ny, int nz, int storage, LaunchCfg even, LaunchCfg odd);
-// One step of many instances in one persistent launch (FP32 populations, the
-// instances' flag bytes required); units: {instance, first, count, -} with
-// first/count in two-cell vectors (parity 0) or cells (parity 1).  stats != 0 writes NSTAT sums per unit into partials.
 // Two steps, an odd one and the even one behind it, from fa to fb (FP32; parity 1
 // before and after, the whole grid, no macro fields or statistics; solid cells of fb
 // are left as they are).
@@ -91,6 +88,10 @@ cudaError_t launch_pair_solids(const AAParams& p, const float* fa, float* fb, cu
 int pair_zchunk(int nx, int ny, int nz, int storage, bool mask);
 // sets the dynamic shared-memory limit of its kernels (call outside graph capture)
 cudaError_t pair_prepare();
+// One step of many instances in one persistent launch (FP32, F16 or BF16 populations, the
+// instances' flag bytes required); units: {instance, first, count, width} with first/count
+// in vectors of `width` cells (parity 0) or cells (parity 1).  stats != 0 writes NSTAT sums
+// per unit into partials.
 cudaError_t launch_aa_batch(const AAParams* d_inst, const int4* d_units, int nunits, int parity, int stats,
                             int storage, int blocks, int threads, double* partials, cudaStream_t s);
 // per-instance sums of the unit partials: units of instance i are first[i]..first[i+1]-1
