@@ -112,3 +112,22 @@ def test_passes_are_reported_as_they_are_taken(gpu, make, pairs):
             assert told == n if not pairs or n < 4 else told <= n
         assert s.step_passes(50) == (26 if pairs else 50)      # (an even parity, with macro fields 1 + 24 + 1)
     s.close()
+
+
+def test_buffer_is_taken_while_a_stream_captures(gpu):
+    """An instance of a batch holds no buffer: its own call takes it, captured by the caller or by step_graph."""
+    for captured in (True, False):
+        a, b, one = [Solver(*DIMS, 0.6) for _ in range(3)]
+        batch = Batch([a, b])
+        if captured:
+            assert launches(a, 9) == 7      # (1 + 2 + 4: not run, the host's parity is odd now)
+            a.step(1)
+        else:
+            for s in (a, one):
+                s.step_graph(9)
+                s.step_graph(9)
+            np.testing.assert_array_equal(a.state(), one.state())
+        assert a.step_passes(50) == 26
+        a.synchronize()
+        for s in (batch, a, b, one):
+            s.close()
